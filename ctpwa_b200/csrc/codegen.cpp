@@ -1119,6 +1119,169 @@ std::string Gen::emit()
          "    float* dFr, float* dFi)\n{\n"
          "  (void)evf; (void)evd; (void)C; (void)Cfh; (void)Cfl; (void)dFr; (void)dFi;\n"
       << callPart(true) << "}\n";
+    // ---------------- one-pass Hessian form ----------------
+    // The FP64 lineshape values, first and second theta derivatives as one
+    // straight-line function that hands each result to a sink as soon as it
+    // is formed (the kernel consumes the derivatives at once, so few of them
+    // are live together): s.value(t, re, im) for every term, s.sums(), then
+    // per term its first derivatives s.der(k, t, row, re, im) and second
+    // derivatives s.second(m, t, row, re, im); `row` numbers the event's
+    // linear Hessian sums (two for a first derivative, one for a second) in
+    // that order. Second derivatives multiply event-only factors the
+    // frontier may hold only separately; such products are formed here from
+    // frontier values. If one needs a value below the frontier the model has
+    // no one-pass form. Last: it adds nodes to the graph.
+    {
+        struct D2 {
+            int term, j0, j1, re, im;
+        };
+        std::vector<D2> d2;
+        for (size_t t = 0; t < cols.size(); ++t) {
+            const auto der = cols[t].der;
+            for (size_t i = 0; i < der.size(); ++i)
+                for (size_t j = i; j < der.size(); ++j) {
+                    const int re = G.deriv(der[i].second.first, der[j].first),
+                              im = G.deriv(der[i].second.second, der[j].first);
+                    if (G.isConst(re) && G.val(re) == 0.0 && G.isConst(im) && G.val(im) == 0.0) continue;
+                    d2.push_back({(int)t, der[i].first, der[j].first, re, im});
+                }
+        }
+        const size_t n = N.size();
+        std::vector<char> hlive(n, 0);
+        std::vector<int> st;
+        for (const auto& c : cols) {
+            st.push_back(c.re);
+            st.push_back(c.im);
+            for (const auto& d : c.der) {
+                st.push_back(d.second.first);
+                st.push_back(d.second.second);
+            }
+        }
+        for (const auto& d : d2) {
+            st.push_back(d.re);
+            st.push_back(d.im);
+        }
+        const std::vector<int> hroots = st;
+        auto inFrontier = [&](int x) { return x < (int)fs64.size() && fs64[x] >= 0; };
+        auto hEvOnly = [&](int x) { return N[x].dep == dag::DEP_EVENT && N[x].op != dag::Const; };
+        bool ok = true;
+        while (!st.empty()) {
+            const int x = st.back();
+            st.pop_back();
+            if (x < 0 || hlive[x]) continue;
+            hlive[x] = 1;
+            if (hEvOnly(x) && inFrontier(x)) continue;  // read from the table
+            if (N[x].op == dag::Kin) ok = false;
+            for (int k : {N[x].a, N[x].b, N[x].c})
+                if (k >= 0) st.push_back(k);
+        }
+        // parameter-only constants read per event
+        std::vector<int> hslot(n, -1);
+        int nh = 0;
+        std::vector<char> need(n, 0);
+        for (size_t x = 0; x < n; ++x) {
+            if (!hlive[x] || !(N[x].dep & dag::DEP_EVENT) || (hEvOnly((int)x) && inFrontier((int)x))) continue;
+            for (int k : {N[x].a, N[x].b, N[x].c})
+                if (k >= 0 && N[k].dep == dag::DEP_THETA) need[k] = 1;
+        }
+        for (int r : hroots)
+            if (r >= 0 && N[r].dep == dag::DEP_THETA) need[r] = 1;
+        for (size_t x = 0; x < n; ++x)
+            if (need[x]) hslot[x] = nh++;
+        if (ok) {
+            std::ostringstream hp, hc;
+            for (size_t x = 0; x < n; ++x) {
+                const auto& nd = N[x];
+                if (!hlive[x] || nd.op == dag::Const || nd.dep != dag::DEP_THETA) continue;
+                if (nd.op != dag::Theta)
+                    hp << "  const double t" << x << " = "
+                       << opExpr(nd, nd.a >= 0 ? proRef(nd.a) : "", nd.b >= 0 ? proRef(nd.b) : "",
+                                 nd.c >= 0 ? proRef(nd.c) : "", false)
+                       << ";\n";
+                if (hslot[x] >= 0) hp << "  C[" << hslot[x] << "] = " << proRef((int)x) << ";\n";
+            }
+            auto ref = [&](int x) -> std::string {
+                const auto& nd = N[x];
+                if (nd.op == dag::Const) return num(nd.v);
+                if (nd.dep == dag::DEP_THETA) return "C[" + std::to_string(hslot[x]) + "]";
+                if (hEvOnly(x) && inFrontier(x)) return "ev[" + std::to_string(fs64[x]) + "]";
+                return "e" + std::to_string(x);
+            };
+            std::vector<char> done(n, 0);
+            // the definitions that the nodes `rs` still need, in index order
+            auto define = [&](std::initializer_list<int> rs) {
+                std::vector<int> todo, stk(rs);
+                while (!stk.empty()) {
+                    const int x = stk.back();
+                    stk.pop_back();
+                    if (x < 0 || done[x] || !(N[x].dep & dag::DEP_EVENT) || (hEvOnly(x) && inFrontier(x))) continue;
+                    done[x] = 1;
+                    todo.push_back(x);
+                    for (int k : {N[x].a, N[x].b, N[x].c}) stk.push_back(k);
+                }
+                std::sort(todo.begin(), todo.end());
+                for (int x : todo) {
+                    const auto& nd = N[x];
+                    hc << "  const double e" << x << " = "
+                       << opExpr(nd, nd.a >= 0 ? ref(nd.a) : "", nd.b >= 0 ? ref(nd.b) : "", nd.c >= 0 ? ref(nd.c) : "",
+                                 false)
+                       << ";\n";
+                }
+            };
+            for (size_t t = 0; t < cols.size(); ++t) {
+                define({cols[t].re, cols[t].im});
+                hc << "  s.value(" << t << ", " << ref(cols[t].re) << ", " << ref(cols[t].im) << ");\n";
+            }
+            hc << "  s.sums();\n";
+            std::vector<int> rder, rd2;
+            int row = 0, k = 0;
+            for (size_t t = 0; t < cols.size(); ++t) {
+                for (const auto& d : cols[t].der) {
+                    define({d.second.first, d.second.second});
+                    hc << "  s.der(" << k++ << ", " << t << ", " << row << ", " << ref(d.second.first) << ", "
+                       << ref(d.second.second) << ");\n";
+                    rder.push_back(row);
+                    row += 2;
+                }
+                for (size_t m2 = 0; m2 < d2.size(); ++m2) {
+                    if (d2[m2].term != (int)t) continue;
+                    define({d2[m2].re, d2[m2].im});
+                    hc << "  s.second(" << m2 << ", " << t << ", " << row << ", " << ref(d2[m2].re) << ", "
+                       << ref(d2[m2].im) << ");\n";
+                    rd2.push_back(row++);
+                }
+            }
+            std::ostringstream hh;
+            auto tab = [&](const char* name, const std::vector<int>& v) {
+                hh << "__device__ __forceinline__ int " << name << "(int i) {\n  switch (i) {\n";
+                for (size_t i = 0; i < v.size(); ++i) hh << "  case " << i << ": return " << v[i] << ";\n";
+                hh << "  default: return 0;\n  }\n}\n";
+            };
+            std::vector<int> dt, d0, d1;
+            for (const auto& d : d2) {
+                dt.push_back(d.term);
+                d0.push_back(d.j0);
+                d1.push_back(d.j1);
+            }
+            hh << "// generated by ctpwa_b200 codegen: lineshape products with first and second theta derivatives\n"
+                  "#pragma once\n#define M_ND2 "
+               << d2.size() << "\n#define M_NHC " << nh << "\n#define M_HLIN " << row << "\n";
+            tab("d2_term", dt);
+            tab("d2_th0", d0);
+            tab("d2_th1", d1);
+            tab("hrow_der", rder);
+            tab("hrow_d2", rd2);
+            hh << "__device__ __forceinline__ void hs_prologue(const double* __restrict__ th, double* __restrict__ C)\n{\n"
+                  "  (void)th; (void)C;\n"
+               << hp.str() << "}\n"
+               << "template <class S>\n__device__ __forceinline__ void hs_columns(const double* __restrict__ ev,\n"
+                  "    const double* __restrict__ C, S& s)\n{\n  (void)ev; (void)C;\n"
+               << hc.str() << "}\n";
+            out.hess_header = hh.str();
+            out.nhlin = row;
+            out.nhconst = nh;
+        }
+    }
     return h.str();
 }
 

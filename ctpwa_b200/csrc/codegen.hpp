@@ -25,6 +25,12 @@ struct KinSlot {
 struct GeneratedModel {
     std::string header;          // model.cuh text
     std::string dual_header;     // model_dual.cuh text: the lineshapes in dual numbers (Hessian)
+    // model_hess.cuh text: the lineshapes with their first and second theta
+    // derivatives (one-pass Hessian); empty when a second derivative needs a
+    // per-event value that does not follow from the frontier values
+    std::string hess_header;
+    int nhlin = 0;               // linear Hessian sums per event (M_HLIN)
+    int nhconst = 0;             // parameter-only subexpressions of hess_header
     std::vector<KinSlot> slots;  // kinematic cache layout
     int nplane = 0;              // angular planes = sum over groups of nSL
     int npol = 1;                // polarisation states per plane

@@ -1070,6 +1070,9 @@ Engine::~Engine()
     devFree(d_hrows_);
     devFree(d_hvsums_);
     devFree(d_htsums_);
+    devFree(d_hess_img_);
+    devFree(d_hess_rows_);
+    devFree(d_hess_sums_);
     devFree(d_gpart_);
     devFree(d_npart_);
     devFree(d_nmat_);
@@ -1080,6 +1083,7 @@ Engine::~Engine()
         cudaStreamDestroy(mem_stream_);
     }
     if (hvp_lib_) cudaLibraryUnload((cudaLibrary_t)hvp_lib_);
+    if (hess_lib_) cudaLibraryUnload((cudaLibrary_t)hess_lib_);
     if (gram_lib_) cudaLibraryUnload((cudaLibrary_t)gram_lib_);
     if (gram_hess_lib_) cudaLibraryUnload((cudaLibrary_t)gram_hess_lib_);
     if (norm_lib_) cudaLibraryUnload((cudaLibrary_t)norm_lib_);
@@ -2041,6 +2045,45 @@ std::string jitHvpCubin(const GeneratedModel& gen, bool paired, bool* cache_hit)
                       optv, "Hessian kernel", cache_hit);
 }
 
+// Launch of the one-pass Hessian kernel (kernels/hessgram.cuh): blocks of 8
+// rows of the matrix, warps per CTA, minimum resident CTAs per SM, doubles of
+// one CTA row and dynamic shared memory. blocks == 0: the model has no
+// one-pass form, or its matrix has more than 48 rows (21 blocks of
+// accumulators, 84 registers a thread).
+struct HessShape {
+    int blocks = 0, warps = 4, minb = 2, row = 0, dsmem = 0;
+};
+HessShape hessShape(const GeneratedModel& gen)
+{
+    HessShape h;
+    const int hp = gen.ngrad, hb = (hp + 7) / 8;
+    if (gen.hess_header.empty() || hp < 1 || hb > 6) return h;
+    h.blocks = hb;
+    h.row = hb * (hb + 1) / 2 * 64 + gen.nhlin + 1;
+    const int slab = std::max(std::max(8 * hb * 68, 32 * 33), h.row);
+    h.dsmem = h.warps * slab * (int)sizeof(double);
+    if (h.dsmem > 110 * 1024) h.minb = 1;
+    if (h.dsmem > 220 * 1024) h.blocks = 0;
+    return h;
+}
+
+// The one-pass Hessian kernels of one generated model.
+std::string jitHessCubin(const GeneratedModel& gen, bool paired, bool* cache_hit)
+{
+    std::string dir = kernelDir();
+    const HessShape h = hessShape(gen);
+    std::vector<std::string> optv = kNvrtcBase;
+    optv.push_back("-DCT_HESS_WARPS=" + std::to_string(h.warps));
+    optv.push_back("-DCT_HESS_MINB=" + std::to_string(h.minb));
+    optv.push_back(std::string("-DCT_HESS_PAIRED=") + (paired ? "1" : "0"));
+    return nvrtcCubin("#include \"hessgram.cuh\"\n",
+                      {{"device_helpers.cuh", readFile(dir + "/device_helpers.cuh")},
+                       {"hessgram.cuh", readFile(dir + "/hessgram.cuh")},
+                       {"model.cuh", gen.header},
+                       {"model_hess.cuh", gen.hess_header}},
+                      optv, "one-pass Hessian kernel", cache_hit);
+}
+
 // The tensor-core Gram kernels of one generated model (kernels/gram.cuh).
 std::string jitGramCubin(const GeneratedModel& gen, bool paired, bool* cache_hit, bool hess = false)
 {
@@ -2157,6 +2200,14 @@ double precompileConfig(const std::string& config_path)
     bool hit = false;
     jitCubin(g, &hit);
     jitHvpCubin(g, false, &hit);
+    if (hessShape(g).blocks) {
+        if (const char* out = std::getenv("CTPWA_MODEL_SOURCE_OUT"); out && *out) {
+            std::ofstream f(std::string(out) + ".hess.cuh");
+            f << g.hess_header;
+        }
+        jitHessCubin(g, false, &hit);
+        jitHessCubin(g, true, &hit);
+    }
     if (g.nterm + g.nder <= 256 && (size_t)(2 * g.nterm + g.nder) * g.nterm * 16 <= 40000) jitNormCubin(g, &hit);
     {
         std::vector<AgNodeVar> vars;
@@ -2735,6 +2786,42 @@ struct CtHvpArgsH {
     int pad;
 };
 
+// argument blocks of the one-pass Hessian kernels (must match kernels/hessgram.cuh)
+struct CtHessSampleH {
+    const double2* slamp;
+    const double* ev;
+    const double* w;
+    long long n;
+    long long ld;
+    int kind;
+    int group;
+    int cta_begin;
+    int cta_count;
+};
+struct CtHessArgsH {
+    CtHessSampleH s[4];
+    int nsamp;
+    int pad;
+    const double* theta;
+    const double* v;
+    void* img;
+    double* rows;
+};
+struct CtHessGroupsH {
+    int beg[4], cnt[4];
+};
+struct CtHessContractArgsH {
+    const double* sums;
+    const double* dirs;
+    int ndir, nparam, nc, weighted;
+    const int* chain;
+    const double* ratio;
+    const double* v;
+    double n_phsp, w_phsp, w_data, w_bkg;
+    double* tsums;
+    double* vsums;
+};
+
 struct HvpFinalizeArgs {
     const double* vsums;  // [3][nacc] + [n_phsp, W_phsp, W_data, W_bkg]
     const double* tsums;  // [ndir][3][nacc]
@@ -2771,13 +2858,12 @@ __global__ void __launch_bounds__(1024) ct_hvp_rowsum_kernel(const double* __res
     }
 }
 
-// One thread per direction u: the directional derivative of the gradient
+// One warp per direction u: the directional derivative of the gradient
 // assembly of ct_finalize_kernel (loss terms, phase-space normalisation,
 // Gaussian constraints, coupling transform), i.e. the row H u.
 __global__ void ct_hvp_finalize_kernel(HvpFinalizeArgs A)
 {
-    const int d = blockIdx.x * blockDim.x + threadIdx.x;
-    if (d >= A.ndir) return;
+    const int d = blockIdx.x, lane = threadIdx.x;
     const int nacc = A.nacc, nP = 2 * A.nc + A.nT;
     const double* P = A.vsums;
     const double* Dd = A.vsums + nacc;
@@ -2803,12 +2889,12 @@ __global__ void ct_hvp_finalize_kernel(HvpFinalizeArgs A)
         loss += dl * dl / (2.0 * A.gauss_ms[2 * g + 1] * A.gauss_ms[2 * g + 1]);
     }
     if (isnan(loss) || isinf(loss)) {
-        for (int k = 0; k < nP; ++k) out[k] = 0.0;
+        for (int k = lane; k < nP; k += 32) out[k] = 0.0;
         return;
     }
     const double s = 1.0 / (Wp > 0 ? Wp : 1.0);
     const double pf2 = pf * pf;
-    for (int c = 0; c < A.nc; ++c) {
+    for (int c = lane; c < A.nc; c += 32) {
         double sr = 0.0, si = 0.0;
         for (int a = 0; a < A.nA; ++a) {
             if (A.chain[a] != c) continue;
@@ -2825,10 +2911,11 @@ __global__ void ct_hvp_finalize_kernel(HvpFinalizeArgs A)
         out[A.nc + c] = -2.0 * (si * pr - sr * pi) / ps;
     }
     const int j0 = 2 + 2 * A.nA;
-    for (int j = 0; j < A.nT; ++j)
+    for (int j = lane; j < A.nT; j += 32)
         out[2 * A.nc + j] =
             TD[j0 + j] - TB[j0 + j] + (Weff / n_phsp) * (TP[j0 + j] / pf - P[j0 + j] * pft / pf2);
-    for (int g = 0; g < A.ngauss; ++g) {
+    __syncwarp();
+    for (int g = 0; g < A.ngauss && lane == 0; ++g) {
         const int j = A.gauss_idx[g];
         out[2 * A.nc + j] += u[2 * A.nc + j] / (A.gauss_ms[2 * g + 1] * A.gauss_ms[2 * g + 1]);
     }
@@ -2842,9 +2929,41 @@ __global__ void ct_identity_kernel(double* __restrict__ I, int n)
 
 }  // namespace
 
+// A first call may come while the caller's stream is being captured (a
+// Hessian after Hessian-vector products, or the reverse): loading the kernels
+// and allocating then needs this thread's capture checks relaxed. None of
+// that work goes to the captured stream.
+struct RelaxedCapture {
+    cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+    RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+    ~RelaxedCapture() { cudaThreadExchangeStreamCaptureMode(&mode); }
+};
+
+// Buffers of the Hessian-vector products that both forms use: the unit
+// directions, the value sums and the tangent sums of one batch of directions.
+void Engine::hvpBuffers()
+{
+    if (d_htsums_) return;
+    RelaxedCapture relaxed;
+    const int nP = std::max(1, model_.nParams());
+    const int nacc = 2 + 2 * model_.nAmp() + model_.nTheta();
+    hvp_cap_ = std::max(nP, 32);
+    alloc(d_hdirs_, sizeof(double) * (size_t)nP * nP);
+    alloc(d_hvsums_, sizeof(double) * (size_t)sumsSize());
+    cudaStream_t st;
+    CT_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
+    ct_identity_kernel<<<std::max(1, std::min(1024, (nP * nP + 255) / 256)), 256, 0, st>>>(d_hdirs_, nP);
+    CT_CUDA(cudaGetLastError());
+    CT_CUDA(cudaStreamSynchronize(st));
+    cudaStreamDestroy(st);
+    alloc(d_htsums_, sizeof(double) * (size_t)hvp_cap_ * 3 * nacc);
+}
+
 void Engine::compileHvp()
 {
+    hvpBuffers();
     if (k_hvp_) return;
+    RelaxedCapture relaxed;
     bool hit = false;
     std::string cubin = jitHvpCubin(gen_, paired_[0], &hit);
     cudaLibrary_t lib;
@@ -2865,24 +2984,151 @@ void Engine::compileHvp()
     long long tot = 0;
     for (int k = 0; k < 3; ++k) tot += samples_[k].n;
     layoutCtas(sms * occ, tot, hvp_block_, hlay_);
-    const int nP = std::max(1, model_.nParams());
-    hvp_cap_ = std::max(nP, 32);
-    alloc(d_hdirs_, sizeof(double) * (size_t)nP * nP);
     alloc(d_hconsts_, sizeof(double) * 2 * (size_t)hvp_cap_ * std::max(1, gen_.nconst));
     alloc(d_hrows_, sizeof(double) * (size_t)hvp_cap_ * hlay_.grid * nacc);
-    alloc(d_hvsums_, sizeof(double) * (size_t)sumsSize());
-    alloc(d_htsums_, sizeof(double) * (size_t)hvp_cap_ * 3 * nacc);
-    cudaStream_t st;
-    CT_CUDA(cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking));
-    ct_identity_kernel<<<std::max(1, std::min(1024, (nP * nP + 255) / 256)), 256, 0, st>>>(d_hdirs_, nP);
-    CT_CUDA(cudaGetLastError());
-    CT_CUDA(cudaStreamSynchronize(st));
-    cudaStreamDestroy(st);
     k_hvp_pro_ = (void*)kp;
     k_hvp_ = (void*)kh;
 }
 
+void Engine::compileHess()
+{
+    hvpBuffers();
+    if (k_hess_) return;
+    RelaxedCapture relaxed;
+    const HessShape h = hessShape(gen_);
+    bool hit = false;
+    std::string cubin = jitHessCubin(gen_, paired_[0], &hit);
+    cudaLibrary_t lib;
+    CT_CUDA(cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
+    hess_lib_ = (void*)lib;
+    cudaKernel_t kp, kh, kr, kc;
+    CT_CUDA(cudaLibraryGetKernel(&kp, lib, "ct_hess_prologue"));
+    CT_CUDA(cudaLibraryGetKernel(&kh, lib, "ct_hess_f64"));
+    CT_CUDA(cudaLibraryGetKernel(&kr, lib, "ct_hess_reduce"));
+    CT_CUDA(cudaLibraryGetKernel(&kc, lib, "ct_hess_contract"));
+    CT_CUDA(cudaLibraryGetGlobal(&hess_sym_, &hess_sym_bytes_, lib, "hs_k"));
+    CT_CUDA(cudaFuncSetAttribute((const void*)kh, cudaFuncAttributeMaxDynamicSharedMemorySize, h.dsmem));
+    int sms = 148;
+    CT_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, opt_.device));
+    const int occ = residentCtas((void*)kh, 32 * h.warps, h.dsmem);
+    // one wave of CTAs over the samples; a weighted phase-space sample is
+    // passed over twice (the coupling sums carry its weights, the intensity
+    // and resonance-parameter sums do not)
+    long long n[4] = {samples_[0].n, samples_[1].n, samples_[2].n, samples_[0].w ? samples_[0].n : 0};
+    long long tot = 0;
+    for (long long x : n) tot += x;
+    int begin = 0;
+    for (int k = 0; k < 4; ++k) {
+        const long long most = (n[k] + 32 * h.warps - 1) / (32 * h.warps);
+        long long want = n[k] > 0 ? (long long)std::llround((double)sms * occ * n[k] / tot) : 0;
+        if (n[k] > 0) want = std::max(1LL, std::min(most, want));
+        hess_lay_[k][0] = begin;
+        hess_lay_[k][1] = (int)want;
+        begin += (int)want;
+    }
+    // rounding must not leave CTAs for a second wave
+    for (int over = begin - sms * occ; over > 0; --over) {
+        int big = 0;
+        for (int k = 1; k < 4; ++k)
+            if (hess_lay_[k][1] > hess_lay_[big][1]) big = k;
+        if (hess_lay_[big][1] <= 1) break;
+        --hess_lay_[big][1];
+        for (int k = big + 1; k < 4; ++k) --hess_lay_[k][0];
+        --begin;
+    }
+    hess_grid_ = std::max(1, begin);
+    alloc(d_hess_img_, hess_sym_bytes_);
+    alloc(d_hess_rows_, sizeof(double) * (size_t)hess_grid_ * h.row);
+    alloc(d_hess_sums_, sizeof(double) * 4 * (size_t)h.row);
+    k_hess_pro_ = (void*)kp;
+    k_hess_red_ = (void*)kr;
+    k_hess_con_ = (void*)kc;
+    k_hess_ = (void*)kh;
+}
+
+// The one-pass form costs the same for any number of directions, forward mode
+// a pass per direction: K+K-pi0, 11.1M events, 5.4 ms against 1.3 ms per
+// direction (30.1 ms for all 23); three chains of rho, 1.11M events, 0.62 ms
+// against 0.13 ms (3.2 ms for all 24).
+bool Engine::onePassHessian(int ndir) const { return ndir >= 5 && hessShape(gen_).blocks > 0; }
+
+// The one pass over the events and the contraction with the directions; the
+// value sums of the same pass too when d_vsums is given. d_v_ holds the couplings.
+void Engine::hessSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums, double* d_vsums,
+                      cudaStream_t stream)
+{
+    compileHess();
+    const HessShape h = hessShape(gen_);
+    const Model& m = model_;
+    const int nc = m.nVector();
+    CtHessArgsH a;
+    std::memset(&a, 0, sizeof(a));
+    CtHessGroupsH g;
+    std::memset(&g, 0, sizeof(g));
+    for (int k = 0; k < 4; ++k) {
+        g.beg[k] = hess_lay_[k][0];
+        g.cnt[k] = hess_lay_[k][1];
+        if (hess_lay_[k][1] == 0) continue;
+        CtHessSampleH& sm = a.s[a.nsamp++];
+        const DeviceSample& d = samples_[k % 3];
+        sm.slamp = paired_[0] ? d.slamp64p : d.slamp64;
+        sm.ev = d.ev64;
+        sm.w = k == 0 ? nullptr : d.w;
+        sm.n = d.n;
+        sm.ld = d.ld;
+        sm.kind = k % 3;
+        sm.group = k;
+        sm.cta_begin = hess_lay_[k][0];
+        sm.cta_count = hess_lay_[k][1];
+    }
+    a.theta = d_params + 2 * nc;
+    a.v = d_v_;
+    a.img = d_hess_img_;
+    a.rows = d_hess_rows_;
+    void* args[] = {&a};
+    CT_CUDA(cudaLaunchKernel(k_hess_pro_, dim3(1), dim3(32), args, 0, stream));
+    CT_CUDA(cudaMemcpyAsync(hess_sym_, d_hess_img_, hess_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
+    if (a.nsamp > 0)
+        CT_CUDA(cudaLaunchKernel(k_hess_, dim3(hess_grid_), dim3(32 * h.warps), args, (size_t)h.dsmem, stream));
+    void* rargs[] = {&d_hess_rows_, &g, &d_hess_sums_};
+    CT_CUDA(cudaLaunchKernel(k_hess_red_, dim3((h.row + 31) / 32, 4), dim3(256), rargs, 0, stream));
+    CtHessContractArgsH c;
+    std::memset(&c, 0, sizeof(c));
+    c.sums = d_hess_sums_;
+    c.dirs = d_dirs;
+    c.ndir = ndir;
+    c.nparam = m.nParams();
+    c.nc = nc;
+    c.weighted = hess_lay_[3][1] > 0;
+    c.chain = d_amp_chain_;
+    c.ratio = d_ratio_;
+    c.v = d_v_;
+    c.n_phsp = (double)samples_[0].n;
+    c.w_phsp = samples_[0].wsum;
+    c.w_data = samples_[1].wsum;
+    c.w_bkg = has_bkg_ ? samples_[2].wsum : 0.0;
+    c.tsums = d_tsums;
+    c.vsums = d_vsums;
+    void* cargs[] = {&c};
+    CT_CUDA(cudaLaunchKernel(k_hess_con_, dim3(ndir + (d_vsums ? 1 : 0)), dim3(64), cargs, 0, stream));
+}
+
 void Engine::hvpSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums, cudaStream_t stream)
+{
+    if (ndir <= 0) return;
+    if (!onePassHessian(ndir)) {
+        forwardHvpSums(d_params, d_dirs, ndir, d_tsums, stream);
+        return;
+    }
+    const int nA = model_.nAmp();
+    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, model_.nVector(), d_v_,
+                                                            nullptr);
+    CT_CUDA(cudaGetLastError());
+    hessSums(d_params, d_dirs, ndir, d_tsums, nullptr, stream);
+}
+
+void Engine::forwardHvpSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums,
+                            cudaStream_t stream)
 {
     if (ndir <= 0) return;
     compileHvp();
@@ -2957,7 +3203,7 @@ void Engine::finalizeHvp(const double* d_params, const double* d_dirs, int ndir,
     f.ndir = ndir;
     f.err = d_err_;
     f.out = d_out;
-    ct_hvp_finalize_kernel<<<(ndir + 63) / 64, 64, 0, stream>>>(f);
+    ct_hvp_finalize_kernel<<<ndir, 32, 0, stream>>>(f);
     CT_CUDA(cudaGetLastError());
 }
 
@@ -3088,7 +3334,7 @@ void Engine::hessianGram(const double* d_params, double* d_hess, cudaStream_t st
 {
     compileGram();
     compileGramHess();
-    compileHvp();
+    hvpBuffers();
     const Model& m = model_;
     const int nA = m.nAmp(), nc = m.nVector(), nT = m.nTheta(), nP = m.nParams(), NA2 = 2 * nA;
     std::vector<double> hp(nP);
@@ -3503,6 +3749,8 @@ void Engine::gram(const double* d_params, double* d_out, cudaStream_t stream)
     CT_CUDA(cudaLaunchKernel(k_gram_fin_, dim3(1), dim3(256), fargs, 0, stream));
 }
 
+// Forward mode, whatever the number of directions: a direction's product is
+// then the same to the last bit alone and among others.
 void Engine::hessianVectorProducts(const double* d_params, const double* d_dirs, int ndir, double* d_out,
                                    cudaStream_t stream)
 {
@@ -3512,16 +3760,24 @@ void Engine::hessianVectorProducts(const double* d_params, const double* d_dirs,
     for (int d0 = 0; d0 < ndir; d0 += hvp_cap_) {
         const int nd = std::min(hvp_cap_, ndir - d0);
         const size_t off = (size_t)d0 * model_.nParams();
-        hvpSums(d_params, d_dirs + off, nd, d_htsums_, stream);
+        forwardHvpSums(d_params, d_dirs + off, nd, d_htsums_, stream);
         finalizeHvp(d_params, d_dirs + off, nd, d_hvsums_, d_htsums_, d_out + off, stream);
     }
 }
 
 void Engine::hessianExact(const double* d_params, double* d_hess, cudaStream_t stream)
 {
-    compileHvp();
-    const int n = model_.nParams();
-    hessianVectorProducts(d_params, d_hdirs_, n, d_hess, stream);
+    hvpBuffers();
+    const int n = model_.nParams(), nA = model_.nAmp();
+    if (onePassHessian(n)) {
+        ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, model_.nVector(),
+                                                                d_v_, d_err_);
+        CT_CUDA(cudaGetLastError());
+        hessSums(d_params, d_hdirs_, n, d_htsums_, d_hvsums_, stream);
+        finalizeHvp(d_params, d_hdirs_, n, d_hvsums_, d_htsums_, d_hess, stream);
+    } else {
+        hessianVectorProducts(d_params, d_hdirs_, n, d_hess, stream);
+    }
     ct_symmetrize_kernel<<<std::max(1, (n * n + 255) / 256), 256, 0, stream>>>(d_hess, n);
     CT_CUDA(cudaGetLastError());
 }

@@ -225,6 +225,25 @@ private:
     void* k_pc_[2] = {nullptr, nullptr};  // ct_fused_f64_pc, ct_fused_mixed_pc
     void compileKernel();
     void compileHvp();
+    void hvpBuffers();
+    void forwardHvpSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums, cudaStream_t stream);
+    // one-pass Hessian sums (kernels/hessgram.cuh; compiled and allocated on first use)
+    void compileHess();
+    bool onePassHessian(int ndir) const;
+    void hessSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums, double* d_vsums,
+                  cudaStream_t stream);
+    void* hess_lib_ = nullptr;
+    void* k_hess_pro_ = nullptr;
+    void* k_hess_ = nullptr;
+    void* k_hess_red_ = nullptr;
+    void* k_hess_con_ = nullptr;
+    void* hess_sym_ = nullptr;  // the module's constant block and its image
+    size_t hess_sym_bytes_ = 0;
+    void* d_hess_img_ = nullptr;
+    int hess_lay_[4][2] = {};   // first CTA and CTAs of phase space, data, background, weighted phase space
+    int hess_grid_ = 0;
+    double* d_hess_rows_ = nullptr;
+    double* d_hess_sums_ = nullptr;
 
     Model model_;
     EngineOptions opt_;

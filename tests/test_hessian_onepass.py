@@ -1,0 +1,99 @@
+"""The one-pass Hessian sums (kernels/hessgram.cuh) against forward mode.
+
+getHessian takes the one pass, getHessianVectorProduct along the unit
+directions recomputes every event in dual numbers; both are FP64 sums of the
+same terms, so they differ by rounding only: 1e-11 of the largest entry (the
+bound the linearity test of the products uses)."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _many_resonances(nres):
+    """Three chains x nres resonances: 3 nres amplitudes, 2 nres free resonance parameters."""
+    from ctpwa_b200 import workloads
+
+    names = [f"r{i}" for i in range(nres)]
+    txt = workloads.config_text("pipi_3rho", "p", "d")
+    txt = txt[:txt.index("Resonances:")].replace("rho770, rho1450, rho1700", ", ".join(names))
+    return txt + "Resonances:\n" + "".join(
+        f"  {n}: {{J: 1, P: -1, model: BWR, parameters: [{0.8 + 0.13 * i:.3f}, {0.15 + 0.02 * i:.3f}], free: [0, 1]}}\n"
+        for i, n in enumerate(names))
+
+
+def _compare(tmp_path, text, masses, sizes, weights=(False, False, False), seed=1):
+    import torch
+
+    import ctpwa_b200
+    from ctpwa_b200 import toymc, workloads
+
+    cfg = tmp_path / "c.yml"
+    cfg.write_text(text)
+    rng = np.random.default_rng(seed)
+    dev = "cuda:0"
+    s = [torch.tensor(toymc.phase_space(workloads.M_JPSI, masses, n, 100 + seed + k), device=dev) if n else None
+         for k, n in enumerate(sizes)]
+    # signed weights: data and background events of negative weight enter with the opposite sign, zero drops out
+    w = [torch.tensor(np.where(np.arange(n) % 7 == 3, 0.0, rng.uniform(0.5 if k == 0 else -0.4, 1.5, n)), device=dev)
+         if use else None for k, (n, use) in enumerate(zip(sizes, weights))]
+    ana = ctpwa_b200.analysis.from_device(str(cfg), s[0], s[1], s[2], weights=w)
+    p = torch.tensor(workloads.true_params(ana.getNVector(), ana.getFreeResParams()[0].numpy(), seed=seed) *
+                     rng.uniform(0.97, 1.03, ana.getNParams()), device=dev)
+    H = ana.getHessian(p)
+    F = ana.getHessianVectorProduct(p, torch.eye(p.numel(), dtype=torch.float64, device=dev))
+    F = 0.5 * (F + F.T)
+    assert torch.isfinite(F).all() and float(F.abs().max()) > 0
+    assert float((H - F).abs().max()) <= 1e-11 * float(F.abs().max())
+    assert torch.equal(H, ana.getHessian(p))  # fixed summation order
+
+
+@pytest.mark.parametrize("sizes", [(1, 1, 0), (31, 33, 1), (32, 32, 32), (129, 127, 63), (40_000, 4_001, 395)])
+def test_tile_edges(tmp_path, sizes):
+    from ctpwa_b200 import workloads
+
+    _compare(tmp_path, workloads.config_text("kkpi", "p", "d"), workloads.MASSES["kkpi"], sizes)
+
+
+@pytest.mark.parametrize("model", ["pipi_rho", "pipi_3rho", "ksks", "kkpi"])
+@pytest.mark.parametrize("paired", [True, False])
+def test_models_and_weights(tmp_path, monkeypatch, model, paired):
+    from ctpwa_b200 import workloads
+
+    if not paired:
+        monkeypatch.setenv("CTPWA_NO_POL_PAIRING", "1")
+    _compare(tmp_path, workloads.config_text(model, "p", "d"), workloads.MASSES[model], (3001, 517, 130),
+             weights=(True, True, True), seed=3)
+
+
+@pytest.mark.parametrize("nres", [6, 7])
+def test_largest_matrix_and_beyond(tmp_path, nres):
+    """48 rows, the largest matrix of the one-pass kernel, and 56, which takes forward mode."""
+    from ctpwa_b200 import workloads
+
+    _compare(tmp_path, _many_resonances(nres), workloads.MASSES["pipi_3rho"], (2000, 300, 40), seed=5)
+
+
+def test_capture_of_the_first_call(tmp_path):
+    """A first getHessian inside a graph capture, after products on the same handle, replays to the eager result."""
+    import torch
+
+    import ctpwa_b200
+    from ctpwa_b200 import toymc, workloads
+
+    cfg = tmp_path / "c.yml"
+    cfg.write_text(workloads.config_text("pipi_rho", "p", "d"))
+    s = [torch.tensor(toymc.phase_space(workloads.M_JPSI, workloads.MASSES["pipi_rho"], n, n), device="cuda:0")
+         for n in (2000, 300)]
+    ana = ctpwa_b200.analysis.from_device(str(cfg), *s)
+    p = torch.tensor(workloads.true_params(ana.getNVector(), ana.getFreeResParams()[0].numpy()), device="cuda:0")
+    ana.getHessianVectorProduct(p, torch.ones_like(p))
+    ana.getNLL(p)
+    torch.cuda.synchronize()
+    g = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(g):
+        H = ana.getHessian(p)
+    p.mul_(1.01)
+    g.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(H, ana.getHessian(p))
