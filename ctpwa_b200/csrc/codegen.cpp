@@ -1038,13 +1038,148 @@ std::string Gen::emit()
         out.dual_header = dh.str();
     }
 
+    // ---------------- adjoint form (fused likelihood kernels) ----------------
+    // Per event the kernel needs sum_t Re(dF_t/dtheta_j W_t), not the
+    // derivatives themselves. Reverse mode through the lineshape values gives
+    // it at about twice the cost of the values, whatever the number of
+    // parameters: the seeds (Re W_t, -Im W_t) are propagated to the
+    // parameter-only constants C_k the values read, whose adjoints are summed
+    // over the events; the CTA then forms the theta sums with the Jacobian
+    // dC_k/dtheta_j, evaluated once per call. As a function with a sink:
+    // s.value(t, re, im) per term, s.sums() (false: the event has no
+    // gradient), then s.adj(k, x) per constant with the seeds s.wr(t),
+    // s.wi(t). A value that selects between branches per event passes its
+    // adjoint to the selected one and zero to the other, which is safe while
+    // the nodes that only such a branch reaches are sums and products (a
+    // reciprocal or a root there may be infinite where it is not selected);
+    // otherwise the model keeps the symbolic derivatives, and the adjoints
+    // are the theta sums themselves. So does the mixed form, for every model:
+    // reverse mode takes it from 870 to 796 instructions per K+K-pi0 event
+    // but from 43.7 to 50.6 us (1.11M events), its chains being longer and
+    // the adjoint sums four registers more (FP64: 93.0 to 86.8 us).
+    std::vector<int> adjConst;              // nodes of the summed adjoints
+    bool reverse = true;
+    {
+        // nodes reached from the outputs without going into a branch
+        std::vector<char> plain(N.size(), 0);
+        std::vector<int> st;
+        for (const auto& c : cols)
+            for (int r : {c.re, c.im}) st.push_back(r);
+        while (!st.empty()) {
+            const int x = st.back();
+            st.pop_back();
+            if (x < 0 || plain[x]) continue;
+            plain[x] = 1;
+            if (N[x].op == dag::Sel) {
+                st.push_back(N[x].c);
+                continue;
+            }
+            for (int k : {N[x].a, N[x].b, N[x].c}) st.push_back(k);
+        }
+        for (size_t x = 0; x < N.size(); ++x) {
+            if (!live[x] || !valueNode[x] || !mixedDep((int)x)) continue;
+            const dag::Op op = N[x].op;
+            if (op == dag::Atan2) reverse = false;
+            if (!plain[x] && op != dag::Add && op != dag::Sub && op != dag::Mul && op != dag::Neg && op != dag::Sel)
+                reverse = false;
+        }
+    }
+    if (reverse) {
+        std::vector<char> used(N.size(), 0);
+        for (const auto& c : cols)
+            for (int r : {c.re, c.im})
+                if (r >= 0 && isTheta(r)) used[r] = 1;
+        for (size_t x = 0; x < N.size(); ++x) {
+            if (!live[x] || !valueNode[x] || !mixedDep((int)x) || N[x].op == dag::RhoRe || N[x].op == dag::RhoIm) continue;
+            for (int k : {N[x].a, N[x].b})
+                if (k >= 0 && isTheta(k)) used[k] = 1;
+        }
+        for (size_t x = 0; x < used.size(); ++x)
+            if (used[x]) adjConst.push_back((int)x);
+    }
+    const int nadj = reverse ? (int)adjConst.size() : m.nTheta();
+    std::vector<int> adjOf(N.size(), -1);
+    for (size_t k = 0; k < adjConst.size(); ++k) adjOf[adjConst[k]] = (int)k;
+    auto adjointPart = [&](bool f32) -> std::string {
+        std::ostringstream os;
+        const RefFn ref = colRef(f32);
+        const bool rev = reverse && !f32;
+        for (size_t x = 0; x < N.size(); ++x)
+            if (live[x] && mixedDep((int)x) && (valueNode[x] || !rev)) os << nodeLine(x, f32, ref);
+        for (size_t t = 0; t < cols.size(); ++t)
+            os << "  s.value(" << t << ", " << ref(cols[t].re, f32) << ", " << ref(cols[t].im, f32) << ");\n";
+        os << "  if (!s.sums()) return;\n";
+        if (!rev) {
+            for (size_t t = 0; t < cols.size(); ++t)
+                for (const auto& d : cols[t].der)
+                    os << "  s.adj(" << d.first << ", " << ref(d.second.first, f32) << " * s.wr(" << t << ") - "
+                       << ref(d.second.second, f32) << " * s.wi(" << t << "));\n";
+            return os.str();
+        }
+        std::vector<std::string> acc(N.size());
+        auto give = [&](int x, const std::string& v) {
+            if (x < 0 || !(N[x].dep & dag::DEP_THETA)) return;
+            if (!mixedDep(x) && adjOf[x] < 0) return;
+            acc[x] += (acc[x].empty() ? "" : " + ") + v;
+        };
+        for (size_t t = 0; t < cols.size(); ++t) {
+            give(cols[t].re, "s.wr(" + std::to_string(t) + ")");
+            give(cols[t].im, "(-s.wi(" + std::to_string(t) + "))");
+        }
+        for (size_t x = N.size(); x-- > 0;) {
+            if (acc[x].empty() || !mixedDep((int)x)) continue;
+            const auto& nd = N[x];
+            const std::string g = "a" + std::to_string(x), n = "e" + std::to_string(x);
+            os << "  const double " << g << " = " << acc[x] << ";\n";
+            const std::string A = nd.a >= 0 ? ref(nd.a, false) : "", B = nd.b >= 0 ? ref(nd.b, false) : "";
+            switch (nd.op) {
+            case dag::Add:
+                give(nd.a, g);
+                give(nd.b, g);
+                break;
+            case dag::Sub:
+                give(nd.a, g);
+                give(nd.b, "(-" + g + ")");
+                break;
+            case dag::Mul:
+                if (nd.a == nd.b) {
+                    give(nd.a, "(2.0 * " + g + ") * " + A);
+                } else {
+                    give(nd.a, g + " * " + B);
+                    give(nd.b, g + " * " + A);
+                }
+                break;
+            case dag::Recip: give(nd.a, "(-" + g + ") * (" + n + " * " + n + ")"); break;
+            case dag::Neg: give(nd.a, "(-" + g + ")"); break;
+            case dag::Sqrt: give(nd.a, "(0.5 * " + g + ") / " + n); break;
+            case dag::Log: give(nd.a, g + " / " + A); break;
+            case dag::Exp: give(nd.a, g + " * " + n); break;
+            case dag::Sin: give(nd.a, g + " * cos(" + A + ")"); break;
+            case dag::Cos: give(nd.a, "(-" + g + ") * sin(" + A + ")"); break;
+            case dag::Sel: {
+                static const char* ops[] = {">=", ">", "<=", "<", "=="};
+                const std::string c = "(" + ref(nd.c, false) + " " + ops[nd.cmp] + " 0.0";
+                give(nd.a, c + " ? " + g + " : 0.0)");
+                give(nd.b, c + " ? 0.0 : " + g + ")");
+                break;
+            }
+            default: break;  // channel factors and table lookups: no theta derivative
+            }
+        }
+        for (size_t k = 0; k < adjConst.size(); ++k)
+            if (!acc[adjConst[k]].empty()) os << "  s.adj(" << k << ", " << acc[adjConst[k]] << ");\n";
+        return os.str();
+    };
+    const std::string adj64 = adjointPart(false), adj32 = adjointPart(true);
+
     std::vector<std::pair<int, int>> der_entries;  // (term, theta)
     for (size_t a = 0; a < cols.size(); ++a)
         for (const auto& d : cols[a].der) der_entries.push_back({(int)a, d.first});
     const int k = (int)der_entries.size();
     out.nder = k;
     out.nterm = (int)cols.size();
-    out.nconst = ncon;
+    out.nsum[0] = 2 * m.nAmp() + nadj;
+    out.nsum[1] = 2 * m.nAmp() + m.nTheta();
     std::ostringstream h;
     auto table = [&](const char* name, const std::vector<int>& v) {
         h << "__device__ __forceinline__ int " << name << "(int i) {\n  switch (i) {\n";
@@ -1054,7 +1189,7 @@ std::string Gen::emit()
     h << "// generated by ctpwa_b200 codegen: model-specific lineshape products\n#pragma once\n";
     h << "#define M_NA " << m.nAmp() << "\n#define M_NTERM " << cols.size() << "\n#define M_NPOL " << m.npol
       << "\n#define M_NPLANE " << out.nplane << "\n#define M_NKIN " << out.slots.size() << "\n#define M_NTH "
-      << m.nTheta() << "\n#define M_NDER " << k << "\n#define M_NCONST " << ncon << "\n";
+      << m.nTheta() << "\n#define M_NDER " << k << "\n#define M_NCONST " << ncon << "\n#define M_NADJ " << nadj << "\n";
     h << "#define M_NEV " << out.nev64 << "\n#define M_NEVF " << out.nevf << "\n#define M_NEVD " << out.nevd << "\n";
     // terms: amplitude column and angular plane of each
     std::vector<int> tcol, tplane;
@@ -1119,6 +1254,61 @@ std::string Gen::emit()
          "    float* dFr, float* dFi)\n{\n"
          "  (void)evf; (void)evd; (void)C; (void)Cfh; (void)Cfl; (void)dFr; (void)dFi;\n"
       << callPart(true) << "}\n";
+    h << "// lineshape values and, from the seeds of the sink, the adjoints of the parameter-only\n"
+         "// constants (FP64; mixed form)\n";
+    h << "template <class S>\n__device__ __forceinline__ void model_adjoint(const double* __restrict__ ev,\n"
+         "    const double* __restrict__ C, S& s)\n{\n  (void)ev; (void)C;\n"
+      << adj64 << "}\n";
+    h << "template <class S>\n__device__ __forceinline__ void model_adjoint_f32(const float* __restrict__ evf,\n"
+         "    const double* __restrict__ evd, const double* __restrict__ C, const float* __restrict__ Cfh,\n"
+         "    const float* __restrict__ Cfl, S& s)\n{\n  (void)evf; (void)evd; (void)C; (void)Cfh; (void)Cfl;\n"
+      << adj32 << "}\n";
+    // ---------------- Jacobian of the adjoint constants ----------------
+    // (adds nodes to the graph, like everything below)
+    {
+        std::vector<int> ent;  // node of each entry
+        std::vector<std::string> lines(m.nTheta());
+        for (int j = 0; j < m.nTheta(); ++j)
+            for (size_t k2 = 0; k2 < adjConst.size(); ++k2) {
+                const int d = G.deriv(adjConst[k2], j);
+                if (G.isConst(d) && G.val(d) == 0.0) continue;
+                lines[j] += (lines[j].empty() ? "" : " + ") + std::string("J[") + std::to_string(ent.size()) + "] * a[" +
+                            std::to_string(k2) + "]";
+                ent.push_back(d);
+            }
+        std::vector<char> jl(N.size(), 0);
+        std::vector<int> st = ent;
+        while (!st.empty()) {
+            const int x = st.back();
+            st.pop_back();
+            if (x < 0 || jl[x]) continue;
+            jl[x] = 1;
+            for (int k2 : {N[x].a, N[x].b, N[x].c})
+                if (k2 >= 0) st.push_back(k2);
+        }
+        std::ostringstream jp;
+        for (size_t x = 0; x < N.size(); ++x) {
+            const auto& nd = N[x];
+            if (!jl[x] || nd.op == dag::Const || nd.op == dag::Theta) continue;
+            jp << "  const double t" << x << " = "
+               << opExpr(nd, nd.a >= 0 ? proRef(nd.a) : "", nd.b >= 0 ? proRef(nd.b) : "", nd.c >= 0 ? proRef(nd.c) : "",
+                         false)
+               << ";\n";
+        }
+        for (size_t i = 0; i < ent.size(); ++i) jp << "  J[" << i << "] = " << proRef(ent[i]) << ";\n";
+        h << "#define M_NJAC " << ent.size() << "\n"
+          << "// Jacobian of the adjoint constants, once per call, and the theta sums from theirs\n"
+             "__device__ __forceinline__ void model_jacobian(const double* __restrict__ th, double* __restrict__ J)\n{\n"
+             "  (void)th; (void)J;\n"
+          << jp.str() << "}\n"
+          << "__device__ __forceinline__ double model_theta_sum(int j, const double* __restrict__ J, const double* a)\n{\n"
+             "  (void)J;\n  switch (j) {\n";
+        for (int j = 0; j < m.nTheta(); ++j)
+            h << "  case " << j << ": return " << (reverse ? (lines[j].empty() ? "0.0" : lines[j]) : "a[" + std::to_string(j) + "]")
+              << ";\n";
+        h << "  default: return 0.0;\n  }\n}\n";
+        out.nconst = ncon + (int)ent.size();
+    }
     // ---------------- one-pass Hessian form ----------------
     // The FP64 lineshape values, first and second theta derivatives as one
     // straight-line function that hands each result to a sink as soon as it

@@ -34,11 +34,12 @@ struct GeneratedModel {
     std::vector<KinSlot> slots;  // kinematic cache layout
     int nplane = 0;              // angular planes = sum over groups of nSL
     int npol = 1;                // polarisation states per plane
-    int ngrad = 0;               // gradient sums per thread: 2 nA + nTheta
+    int ngrad = 0;               // gradient components: 2 nA + nTheta
+    int nsum[2] = {0, 0};        // gradient sums per thread of the plain and the mixed fused kernels
     std::vector<int> group_plane0;
     int nder = 0;
     int nterm = 0;               // lineshape terms (one per amplitude column, more with identical particles)
-    int nconst = 0;              // parameter-only subexpressions kept per call
+    int nconst = 0;              // parameter-only values kept per call (M_NCONST + M_NJAC)
     // per-event frontier tables (parameter-independent values the per-call
     // code reads): FP64 table rows; mixed form FP32 and FP64 rows
     int nev64 = 0;

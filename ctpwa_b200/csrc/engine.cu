@@ -1889,7 +1889,7 @@ FusedShape fusedShape(const GeneratedModel& gen)
     };
     for (int i = 0; i < 2; ++i) {
         // dynamic shared memory = [gradient-sum slots][two tile buffers]
-        long long acc_bytes = sh.acc[i] ? (gen.ngrad * sh.block[i] * accb[i] + 127) / 128 * 128 : 0;
+        long long acc_bytes = sh.acc[i] ? (gen.nsum[i] * sh.block[i] * accb[i] + 127) / 128 * 128 : 0;
         if (!fits(i, acc_bytes)) {
             sh.acc[i] = 0;
             acc_bytes = 0;
@@ -2295,7 +2295,7 @@ void Engine::nllGrad(const double* d_params, double* d_nll, double* d_grad, int 
     a.kblock = d_kblock_;
     if (precision == kMixed && !samples_[0].slamp32) throw std::runtime_error("mixed-precision tables were not built");
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(32), args, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(k_sym_, d_kblock_, k_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
     const size_t slot = ev_begin_.empty() ? 0 : (size_t)(ev_count_ % (long long)ev_begin_.size());
     if (!ev_begin_.empty()) CT_CUDA(cudaEventRecord(ev_begin_[slot], stream));
@@ -2461,7 +2461,7 @@ void Engine::nllGradMulti(const std::vector<Engine*>& es, const std::vector<cons
     CT_CUDA(cudaGetLastError());
     const CtArgsH* dargs = (const CtArgsH*)(db + o_args);
     void* pargs[] = {&dargs};
-    CT_CUDA(cudaLaunchKernel(e0->k_pro_multi_, dim3(nj), dim3(32), pargs, 0, stream));
+    CT_CUDA(cudaLaunchKernel(e0->k_pro_multi_, dim3(nj), dim3(64), pargs, 0, stream));
     const int* doff = (const int*)(db + o_off);
     int njobs = nj;
     void* fargs[] = {&dargs, &doff, &njobs};
@@ -2572,7 +2572,7 @@ void Engine::nllGradStatic(const double* d_params, double* d_nll, double* d_grad
     a.kblock = base + off_k;
     if (precision == kMixed && !samples_[0].slamp32) throw std::runtime_error("mixed-precision tables were not built");
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(32), args, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(k_sym_, base + off_k, k_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
     a.cta_base = 0;
     CT_CUDA(cudaLaunchKernel(precision == kMixed ? k_mixed_ : k_f64_, dim3(lay.grid), dim3(shape_.block[precision == kMixed]),
@@ -2644,7 +2644,7 @@ void Engine::shardSums(const double* d_params, int precision, double* d_sums, cu
     a.kblock = d_kblock_;
     if (precision == kMixed && !samples_[0].slamp32) throw std::runtime_error("mixed-precision tables were not built");
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(32), args, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(k_sym_, d_kblock_, k_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
     a.cta_base = 0;
     CT_CUDA(cudaLaunchKernel(precision == kMixed ? k_mixed_ : k_f64_, dim3(lay.grid), dim3(shape_.block[precision == kMixed]),
@@ -3567,7 +3567,7 @@ double Engine::normCacheBuild(const double* d_params, cudaStream_t stream)
     pa.v = d_v_;
     pa.consts = d_consts_;
     void* pargs[] = {&pa};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(32), pargs, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), pargs, 0, stream));
     const DeviceSample& d = samples_[0];
     CtNormArgsH a;
     std::memset(&a, 0, sizeof(a));
@@ -3651,7 +3651,7 @@ void Engine::nllGradCached(const double* d_params, double* d_nll, double* d_grad
     a.kblock = d_kblock_;
     if (precision == kMixed && !samples_[1].slamp32) throw std::runtime_error("mixed-precision tables were not built");
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(32), args, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(k_sym_, d_kblock_, k_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
     a.cta_base = 0;
     if (ns > 0)
@@ -3728,7 +3728,7 @@ void Engine::gram(const double* d_params, double* d_out, cudaStream_t stream)
     a.err = d_err_;
     a.kblock = d_kblock_;
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(32), args, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
     const DeviceSample& d = samples_[0];
     CtGramArgsH g;
     std::memset(&g, 0, sizeof(g));
@@ -3856,7 +3856,7 @@ void Engine::partialIntegrals(const double* d_params, int kind, double* d_out, c
     a.consts = d_consts_;
     a.err = d_err_;
     void* pargs[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(32), pargs, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), pargs, 0, stream));
     // rows of nb sums in the partials table (nacc >= nA >= nb columns per row available)
     const int nacc = 2 + 2 * nA + m.nTheta();
     const long long cap_rows = (long long)grid_max_ * nacc / std::max(1, nb);
@@ -3893,7 +3893,7 @@ void Engine::exportWeights(const double* d_params, const std::vector<int>& mask,
     a.consts = d_consts_;
     a.err = d_err_;
     void* pargs[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(32), pargs, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), pargs, 0, stream));
     const int* dmask = nullptr;
     if (!mask.empty()) {
         CT_CUDA(cudaMemcpyAsync(d_mask_, mask.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, stream));
@@ -3932,7 +3932,7 @@ void Engine::intensity(const double* d_params, int kind, double* d_out, cudaStre
     a.consts = d_consts_;
     a.err = d_err_;
     void* pargs[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(32), pargs, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), pargs, 0, stream));
     void* args[] = {&a, &d_out};
     int grid = (int)std::min<long long>((d.n + 255) / 256, 148LL * 16);
     CT_CUDA(cudaLaunchKernel(k_int_, dim3(grid), dim3(256), args, 0, stream));

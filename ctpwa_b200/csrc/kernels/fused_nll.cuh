@@ -19,6 +19,11 @@
 //       (straight-line generated code, FP64)
 //   model_columns_f32(...)   the same in the mixed form (FP32 except the
 //       cancellation-prone polynomial parts such as m0^2 - m^2)
+//   model_adjoint(ev, C, sink)   the values alone, then the adjoints of the
+//       M_NADJ parameter-only constants they read (reverse mode);
+//       model_adjoint_f32(...): the values and the derivatives times the seeds
+//   model_jacobian(theta, J), model_theta_sum(j, J, a)   d constants / d theta,
+//       once per call, and the theta gradient sums from the adjoint sums
 //
 // Per event e of a sample (phase space, data or background) the kernel forms
 //   A_{a,p} = F_a * SL_{plane(a),p},   S_p = sum_a v_a A_{a,p},   f = sum_p |S_p|^2
@@ -51,6 +56,10 @@
 #endif
 
 #define CT_NACC (2 + 2 * M_NA + M_NTH)
+// gradient sums of a thread: couplings, then the adjoints of the
+// parameter-only constants (FP64) or the theta sums (mixed form)
+template <typename L>
+constexpr int ct_nsum = 2 * M_NA + (sizeof(L) == 8 ? M_NADJ : M_NTH);
 
 // shared-memory staging of the event tables: 0 off; by per-warp bulk copies
 // 1 the frontier rows, 2 the frontier and angular rows; 3 the frontier values
@@ -94,7 +103,7 @@ struct CtArgs {
     const double* theta;  // fitted resonance parameters
     const double* v;      // couplings, interleaved (re, im) x M_NA
     double* partials;     // [total CTAs][CT_NACC]
-    double* consts;       // [M_NCONST] parameter-only subexpressions of this call
+    double* consts;       // [M_NCONST + M_NJAC] parameter-only subexpressions of this call, Jacobian of the adjoint constants
     int cta_base;         // CTA index of this launch's first block (split launches)
     int pad2;
     int* err;             // set to 1 when a staged copy did not arrive in time
@@ -128,8 +137,9 @@ struct CtConsts {
 };
 __constant__ CtConsts ct_k;
 
-// The parameter-only part of every lineshape (prologue, one thread), then
-// the constant-bank image of this call (one warp).
+// The parameter-only part of every lineshape and the Jacobian of the adjoint
+// constants (prologue, one thread of a warp each), then the constant-bank
+// image of this call (64 threads).
 __device__ __forceinline__ void ct_prologue_body(const CtArgs& A);
 extern "C" __global__ void ct_prologue(CtArgs A)
 {
@@ -142,6 +152,7 @@ extern "C" __global__ void ct_prologue_multi(const CtArgs* __restrict__ jobs) { 
 __device__ __forceinline__ void ct_prologue_body(const CtArgs& A)
 {
     if (threadIdx.x == 0) model_prologue(A.theta, A.consts);
+    if (threadIdx.x == 32) model_jacobian(A.theta, A.consts + M_NCONST);
     __syncthreads();
     if (!A.kblock) return;
     CtConsts* K = (CtConsts*)A.kblock;
@@ -186,11 +197,11 @@ template <typename L, int BLOCK, bool SMEM>
 struct CtAccG;
 template <typename L, int BLOCK>
 struct CtAccG<L, BLOCK, false> {
-    L v[CT_NACC - 2];
+    L v[ct_nsum<L>];
     __device__ __forceinline__ void init(unsigned char*)
     {
 #pragma unroll
-        for (int i = 0; i < CT_NACC - 2; ++i) v[i] = (L)0;
+        for (int i = 0; i < ct_nsum<L>; ++i) v[i] = (L)0;
     }
     __device__ __forceinline__ void add(int i, L x) { v[i] += x; }
     __device__ __forceinline__ L operator[](int i) const { return v[i]; }
@@ -203,34 +214,42 @@ struct CtAccG<L, BLOCK, true> {
     {
         p = (L*)slot + threadIdx.x;
 #pragma unroll
-        for (int i = 0; i < CT_NACC - 2; ++i) p[i * BLOCK] = (L)0;
+        for (int i = 0; i < ct_nsum<L>; ++i) p[i * BLOCK] = (L)0;
     }
     __device__ __forceinline__ void add(int i, L x) { p[i * BLOCK] += x; }
     __device__ __forceinline__ L operator[](int i) const { return p[i * BLOCK]; }
 };
 
 // (the v-gradient sums are scaled by vscale and the theta-gradient sums by
-// tscale on the way out: the per-event factors common to a CTA's sample)
-template <int BLOCK, typename G>
+// tscale on the way out: the per-event factors common to a CTA's sample; the
+// FP64 theta sums come from the adjoint sums and their Jacobian J)
+template <int BLOCK, typename L, typename G>
 __device__ __forceinline__ void ct_block_reduce_store(const double* accd, const G& accg, double* out, double vscale,
-                                                      double tscale)
+                                                      double tscale, const double* __restrict__ J)
 {
-    __shared__ double red[BLOCK / 32][CT_NACC];
+    constexpr int N = 2 + ct_nsum<L>;
+    __shared__ double red[BLOCK / 32][N], sum[N];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
-    for (int i = 0; i < CT_NACC; ++i) {
+    for (int i = 0; i < N; ++i) {
         double x = i < 2 ? accd[i] : (double)accg[i - 2];
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
         if (lane == 0) red[warp][i] = x;
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < CT_NACC; i += BLOCK) {
+    for (int i = threadIdx.x; i < N; i += BLOCK) {
         double x = 0.0;
 #pragma unroll
         for (int w = 0; w < BLOCK / 32; ++w) x += red[w][i];
-        out[i] = i < 2 ? x : (i < 2 + 2 * M_NA ? x * vscale : x * tscale);
+        sum[i] = x;
     }
+    __syncthreads();
+    for (int i = threadIdx.x; i < CT_NACC; i += BLOCK)
+        out[i] = i < 2              ? sum[i]
+                 : i < 2 + 2 * M_NA ? sum[i] * vscale
+                 : sizeof(L) == 4   ? sum[i] * tscale
+                                    : model_theta_sum(i - 2 - 2 * M_NA, J, sum + 2 + 2 * M_NA) * tscale;
 }
 
 // One event's frontier values and its lineshape products: FP64 rows (plain
@@ -261,6 +280,11 @@ struct CtEvent<double> {
                                             double* dFr, double* dFi) const
     {
         model_columns(v, C, Fr, Fi, dFr, dFi);
+    }
+    template <class S>
+    __device__ __forceinline__ void adjoint(const double* C, const float*, const float*, S& s) const
+    {
+        model_adjoint(v, C, s);
     }
 };
 template <>
@@ -295,6 +319,32 @@ struct CtEvent<float> {
     {
         model_columns_f32(f, d, C, Cfh, Cfl, Fr, Fi, dFr, dFi);
     }
+    template <class S>
+    __device__ __forceinline__ void adjoint(const double* C, const float* Cfh, const float* Cfl, S& s) const
+    {
+        model_adjoint_f32(f, d, C, Cfh, Cfl, s);
+    }
+};
+
+// Sink of model_adjoint*: the event's lineshape values and adjoint seeds W_t;
+// `mid` (the coherent sums, the coupling gradient and the seeds; false when
+// the event has no gradient) runs between the values and the adjoints, `add`
+// takes each summed adjoint.
+template <typename L, class Mid, class Add>
+struct CtAdjointSink {
+    Mid& mid;
+    Add& add;
+    L Fr[M_NTERM], Fi[M_NTERM], Wr[M_NTERM], Wi[M_NTERM];
+    __device__ __forceinline__ CtAdjointSink(Mid& m, Add& a) : mid(m), add(a) {}
+    __device__ __forceinline__ void value(int t, L re, L im)
+    {
+        Fr[t] = re;
+        Fi[t] = im;
+    }
+    __device__ __forceinline__ bool sums() { return mid(Fr, Fi, Wr, Wi); }
+    __device__ __forceinline__ L wr(int t) const { return Wr[t]; }
+    __device__ __forceinline__ L wi(int t) const { return Wi[t]; }
+    __device__ __forceinline__ void adj(int k, L x) { add(k, x); }
 };
 
 // Once per event when a sample is loaded: the frontier tables from the
@@ -360,7 +410,7 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
 
     // dynamic shared memory: [gradient-sum slots (ACC_SMEM)][tile buffers (STAGE)]
     extern __shared__ __align__(128) unsigned char ct_dyn[];
-    constexpr unsigned ACC_BYTES = ACC_SMEM ? ((CT_NACC - 2) * BLOCK * sizeof(L) + 127) / 128 * 128 : 0;
+    constexpr unsigned ACC_BYTES = ACC_SMEM ? (ct_nsum<L> * BLOCK * sizeof(L) + 127) / 128 * 128 : 0;
     double accd[2] = {0.0, 0.0};
     CtAccG<L, BLOCK, ACC_SMEM> accg;
     accg.init(ct_dyn);
@@ -389,9 +439,7 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
         // ---- lineshapes with parameter derivatives ----
         CtEvent<L> ev;
         ev.load(ap, bp, ks);
-        L Fr[M_NTERM], Fi[M_NTERM], dFr[M_NDER > 0 ? M_NDER : 1], dFi[M_NDER > 0 ? M_NDER : 1];
-        ev.columns(sC, sCfh, sCfl, Fr, Fi, dFr, dFi);
-
+        auto mid = [&](const L* Fr, const L* Fi, L* Wr, L* Wi) -> bool {
         // ---- coherent sum over amplitudes ----
         // (paired tables: SL_{c,NPOL-1-p} = conj(SL_{c,p}), only the first
         // CT_NPOL_STORED polarisations are stored and read)
@@ -490,7 +538,7 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
             const double we = wts ? __ldg(wts + e) : 1.0;
             if (f == (R)0) {
                 accd[0] += -log(1e-10) * we;
-                return;
+                return false;
             }
             accd[0] += -log((double)f) * we;
             const R inv = (R)(we / (double)f);
@@ -553,7 +601,6 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
             }
         }
         // theta-gradient: Re(v dF_t conj(T)) = Re(dF_t W_t), W_t = v_col(t) conj(T_plane(t))
-        L Wr[M_NTERM], Wi[M_NTERM];
 #pragma unroll
         for (int t = 0; t < M_NTERM; ++t) {
             const int a = term_col(t), c = term_plane(t);
@@ -561,11 +608,11 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
             Wr[t] = vr(a) * tr + vi(a) * ti;
             Wi[t] = vi(a) * tr - vr(a) * ti;
         }
-#pragma unroll
-        for (int k = 0; k < M_NDER; ++k) {
-            const int t = der_term(k);
-            accg.add(2 * M_NA + der_th(k), dFr[k] * Wr[t] - dFi[k] * Wi[t]);
-        }
+        return true;
+        };
+        auto add = [&](int k, L x) { accg.add(2 * M_NA + k, x); };
+        CtAdjointSink<L, decltype(mid), decltype(add)> sink(mid, add);
+        ev.adjoint(sC, sCfh, sCfl, sink);
     };
 
     if constexpr (STAGE == 3) {
@@ -703,8 +750,8 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
         for (long long e = (long long)(cta - S.cta_begin) * BLOCK + threadIdx.x; e < n; e += stride)
             event(e, CtEvent<L>::at(eva, e), evb ? evb + e : nullptr, S.ld, slat(e), S.ld);
     }
-    ct_block_reduce_store<BLOCK>(accd, accg, A.partials + (long long)cta * CT_NACC, kind == 0 ? S.vw_scale : -1.0,
-                                 kind == 0 ? 2.0 : -2.0);
+    ct_block_reduce_store<BLOCK, L>(accd, accg, A.partials + (long long)cta * CT_NACC, kind == 0 ? S.vw_scale : -1.0,
+                                 kind == 0 ? 2.0 : -2.0, A.consts + M_NCONST);
 }
 
 // block size and minimum resident CTAs per SM of the two fused kernels (the
