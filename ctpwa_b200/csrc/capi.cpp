@@ -435,18 +435,29 @@ int ctpwa_finalize_sums(ctpwa_handle* h, const double* d_params, const double* d
 int ctpwa_nll_grad_host(ctpwa_handle* h, const double* params, double* nll, double* grad, int precision, void* stream)
 {
     if (!h || !params || !nll || !grad) return setErr(h, CTPWA_ERR_ARG, "null argument");
+    if (precision != CTPWA_FP64 && precision != CTPWA_MIXED) return setErr(h, CTPWA_ERR_ARG, "precision must be 0 or 1");
     int np = h->eng->nParams();
     cudaStream_t s = (cudaStream_t)stream;
     try {
-        std::memcpy(h->h_pin, params, sizeof(double) * np);
-        if (cudaMemcpyAsync(h->d_params, h->h_pin, sizeof(double) * np, cudaMemcpyHostToDevice, s) != cudaSuccess)
-            throw std::runtime_error("CUDA error: host-to-device copy failed");
         // points at the cached resonance parameters: from the normalisation cache
-        int rc = h->eng->normCacheMatches(params) ? ctpwa_nll_grad_cached(h, h->d_params, h->d_out, h->d_out + 1, precision, stream)
-                                                  : ctpwa_nll_grad(h, h->d_params, h->d_out, h->d_out + 1, precision, stream);
-        if (rc != CTPWA_OK) return rc;
-        if (cudaMemcpyAsync(h->h_pin + np, h->d_out, sizeof(double) * (1 + np), cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
+        const bool cached = h->eng->normCacheMatches(params);
+        if (np <= ctpwa::Engine::kHostParamsMax) {
+            // the parameters travel with the first launch, the result goes
+            // straight to the pinned buffer: no copies (three chains of rho,
+            // 111k events: TODO us)
+            if (cached) h->eng->nllGradCached(h->d_params, h->h_pin + np, h->h_pin + np + 1, precision, s, params);
+            else h->eng->nllGrad(h->d_params, h->h_pin + np, h->h_pin + np + 1, precision, s, params);
+        } else {
+            std::memcpy(h->h_pin, params, sizeof(double) * np);
+            if (cudaMemcpyAsync(h->d_params, h->h_pin, sizeof(double) * np, cudaMemcpyHostToDevice, s) != cudaSuccess)
+                throw std::runtime_error("CUDA error: host-to-device copy failed");
+            int rc = cached ? ctpwa_nll_grad_cached(h, h->d_params, h->d_out, h->d_out + 1, precision, stream)
+                            : ctpwa_nll_grad(h, h->d_params, h->d_out, h->d_out + 1, precision, stream);
+            if (rc != CTPWA_OK) return rc;
+            if (cudaMemcpyAsync(h->h_pin + np, h->d_out, sizeof(double) * (1 + np), cudaMemcpyDeviceToHost, s) != cudaSuccess)
+                throw std::runtime_error(std::string("CUDA error: ") + cudaGetErrorString(cudaGetLastError()));
+        }
+        if (cudaStreamSynchronize(s) != cudaSuccess)
             throw std::runtime_error(std::string("CUDA error: ") + cudaGetErrorString(cudaGetLastError()));
         *nll = h->h_pin[np];
         std::memcpy(grad, h->h_pin + np + 1, sizeof(double) * np);

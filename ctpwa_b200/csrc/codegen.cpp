@@ -20,6 +20,7 @@
 #include <functional>
 #include <map>
 #include <memory>
+#include <set>
 #include <sstream>
 #include <stdexcept>
 #include <tuple>
@@ -499,7 +500,6 @@ std::string Gen::emit()
         if (needC[x]) cslot[x] = ncon++;
 
     // ---------------- parameter-only prologue (FP64) ----------------
-    std::ostringstream pro;
     auto proRef = [&](int x) -> std::string {
         const auto& nd = N[x];
         if (nd.op == dag::Const) return num(nd.v);
@@ -529,18 +529,67 @@ std::string Gen::emit()
         default: return num(nd.v);
         }
     };
-    for (size_t x = 0; x < N.size(); ++x) {
-        if (!live[x] || N[x].op == dag::Const) continue;
-        if (N[x].dep != dag::DEP_THETA) continue;
-        if (N[x].op != dag::Theta) {
-            const auto& nd = N[x];
-            pro << "  const double t" << x << " = "
-                << opExpr(nd, nd.a >= 0 ? proRef(nd.a) : "", nd.b >= 0 ? proRef(nd.b) : "", nd.c >= 0 ? proRef(nd.c) : "",
-                          false)
-                << ";\n";
+    // A prologue as parts that one thread each evaluates, side by side (its
+    // cost is the latency of one dependent FP64 chain with square roots and
+    // divisions): the outputs in order of the theta they depend on, split
+    // evenly over at most 16 parts; a part repeats the subexpressions it
+    // shares with others.
+    struct ProItem {
+        int slot, node;
+        std::string tail;  // appended to the node's value
+    };
+    std::vector<ProItem> proItems;
+    for (size_t x = 0; x < N.size(); ++x)
+        if (cslot[x] >= 0) proItems.push_back({cslot[x], (int)x, ""});
+    auto prologueText = [&](const std::string& name, const std::string& macro, std::vector<ProItem> items) {
+        std::vector<std::set<int>> deps(items.size());
+        for (size_t i = 0; i < items.size(); ++i) {
+            std::set<int> seen;
+            std::vector<int> st = {items[i].node};
+            while (!st.empty()) {
+                const int x = st.back();
+                st.pop_back();
+                if (x < 0 || !seen.insert(x).second) continue;
+                if (N[x].op == dag::Theta) deps[i].insert(N[x].idx);
+                for (int k : {N[x].a, N[x].b, N[x].c}) st.push_back(k);
+            }
         }
-        if (cslot[x] >= 0) pro << "  C[" << cslot[x] << "] = " << proRef((int)x) << ";\n";
-    }
+        std::vector<size_t> order(items.size());
+        for (size_t i = 0; i < order.size(); ++i) order[i] = i;
+        std::stable_sort(order.begin(), order.end(), [&](size_t i, size_t j) {
+            const int a0 = deps[i].empty() ? -1 : *deps[i].begin(), b0 = deps[j].empty() ? -1 : *deps[j].begin();
+            return a0 != b0 ? a0 < b0 : items[i].slot < items[j].slot;
+        });
+        const size_t parts = std::max<size_t>(1, std::min<size_t>(16, (items.size() + 3) / 4));
+        std::ostringstream o;
+        o << "#define " << macro << " " << parts << "\n__device__ __forceinline__ void " << name
+          << "(int part, const double* th, double* C)\n{\n  (void)th; (void)C;\n  switch (part) {\n";
+        for (size_t q = 0; q < parts; ++q) {
+            std::set<int> need;
+            std::vector<int> st;
+            const size_t i0 = q * items.size() / parts, i1 = (q + 1) * items.size() / parts;
+            for (size_t i = i0; i < i1; ++i) st.push_back(items[order[i]].node);
+            while (!st.empty()) {
+                const int x = st.back();
+                st.pop_back();
+                if (x < 0 || N[x].op == dag::Const || N[x].op == dag::Theta || !need.insert(x).second) continue;
+                for (int k : {N[x].a, N[x].b, N[x].c}) st.push_back(k);
+            }
+            o << "  case " << q << ": {\n";
+            for (int x : need) {
+                const auto& nd = N[x];
+                o << "  const double t" << x << " = "
+                  << opExpr(nd, nd.a >= 0 ? proRef(nd.a) : "", nd.b >= 0 ? proRef(nd.b) : "", nd.c >= 0 ? proRef(nd.c) : "",
+                            false)
+                  << ";\n";
+            }
+            for (size_t i = i0; i < i1; ++i)
+                o << "  C[" << items[order[i]].slot << "] = " << proRef(items[order[i]].node) << items[order[i]].tail << ";\n";
+            o << "  break;\n  }\n";
+        }
+        o << "  default: break;\n  }\n}\n";
+        return o.str();
+    };
 
     // ---------------- per-event code ----------------
     // Event nodes come in two kinds. Event-only nodes (kinematic values,
@@ -751,13 +800,13 @@ std::string Gen::emit()
             auto it = seen.find(key);
             if (it == seen.end()) {
                 it = seen.emplace(key, ncon++).first;
+                proItems.push_back({it->second, t, (add ? " + " : " - ") + num(shiftR[xs])});
                 shiftPro += "  C[" + std::to_string(it->second) + "] = C[" + std::to_string(cslot[t]) + "]" +
                             (add ? " + " : " - ") + num(shiftR[xs]) + ";\n";
             }
             shiftSlot[y] = it->second;
         }
     }
-    pro << shiftPro;
     using RefFn = std::function<std::string(int, bool)>;
     // reference to a kinematic leaf, a table lookup or an event node from the
     // once-per-event code, for a consumer evaluated in FP32 (wantF) or FP64
@@ -1187,7 +1236,7 @@ std::string Gen::emit()
         h << "  default: return 0;\n  }\n}\n";
     };
     h << "// generated by ctpwa_b200 codegen: model-specific lineshape products\n#pragma once\n";
-    h << "#define M_NA " << m.nAmp() << "\n#define M_NTERM " << cols.size() << "\n#define M_NPOL " << m.npol
+    h << "#define M_NA " << m.nAmp() << "\n#define M_NPAR " << m.nParams() << "\n#define M_NTERM " << cols.size() << "\n#define M_NPOL " << m.npol
       << "\n#define M_NPLANE " << out.nplane << "\n#define M_NKIN " << out.slots.size() << "\n#define M_NTH "
       << m.nTheta() << "\n#define M_NDER " << k << "\n#define M_NCONST " << ncon << "\n#define M_NADJ " << nadj << "\n";
     h << "#define M_NEV " << out.nev64 << "\n#define M_NEVF " << out.nevf << "\n#define M_NEVD " << out.nevd << "\n";
@@ -1215,10 +1264,6 @@ std::string Gen::emit()
         if (tables[t].empty()) h << "0.0";
         h << "};\n";
     }
-    h << "// parameter-only subexpressions, evaluated once per likelihood call\n";
-    h << "__device__ __forceinline__ void model_prologue(const double* __restrict__ th, double* __restrict__ C)\n{\n"
-         "  (void)th; (void)C;\n"
-      << pro.str() << "}\n";
     h << "// once per event (sample loading): the parameter-independent values the\n"
          "// per-call code reads (frontier), FP64\n";
     h << "__device__ __forceinline__ void model_event(const double* __restrict__ kv, double* __restrict__ o)\n{\n"
@@ -1276,31 +1321,11 @@ std::string Gen::emit()
                             std::to_string(k2) + "]";
                 ent.push_back(d);
             }
-        std::vector<char> jl(N.size(), 0);
-        std::vector<int> st = ent;
-        while (!st.empty()) {
-            const int x = st.back();
-            st.pop_back();
-            if (x < 0 || jl[x]) continue;
-            jl[x] = 1;
-            for (int k2 : {N[x].a, N[x].b, N[x].c})
-                if (k2 >= 0) st.push_back(k2);
-        }
-        std::ostringstream jp;
-        for (size_t x = 0; x < N.size(); ++x) {
-            const auto& nd = N[x];
-            if (!jl[x] || nd.op == dag::Const || nd.op == dag::Theta) continue;
-            jp << "  const double t" << x << " = "
-               << opExpr(nd, nd.a >= 0 ? proRef(nd.a) : "", nd.b >= 0 ? proRef(nd.b) : "", nd.c >= 0 ? proRef(nd.c) : "",
-                         false)
-               << ";\n";
-        }
-        for (size_t i = 0; i < ent.size(); ++i) jp << "  J[" << i << "] = " << proRef(ent[i]) << ";\n";
+        for (size_t i = 0; i < ent.size(); ++i) proItems.push_back({ncon + (int)i, ent[i], ""});
         h << "#define M_NJAC " << ent.size() << "\n"
-          << "// Jacobian of the adjoint constants, once per call, and the theta sums from theirs\n"
-             "__device__ __forceinline__ void model_jacobian(const double* __restrict__ th, double* __restrict__ J)\n{\n"
-             "  (void)th; (void)J;\n"
-          << jp.str() << "}\n"
+          << "// once per call: the parameter-only subexpressions, then the Jacobian of the adjoint constants\n"
+          << prologueText("model_prologue", "M_NPRO", proItems)
+          << "// theta sums from the adjoint sums\n"
           << "__device__ __forceinline__ double model_theta_sum(int j, const double* __restrict__ J, const double* a)\n{\n"
              "  (void)J;\n  switch (j) {\n";
         for (int j = 0; j < m.nTheta(); ++j)
@@ -1379,17 +1404,10 @@ std::string Gen::emit()
         for (size_t x = 0; x < n; ++x)
             if (need[x]) hslot[x] = nh++;
         if (ok) {
-            std::ostringstream hp, hc;
-            for (size_t x = 0; x < n; ++x) {
-                const auto& nd = N[x];
-                if (!hlive[x] || nd.op == dag::Const || nd.dep != dag::DEP_THETA) continue;
-                if (nd.op != dag::Theta)
-                    hp << "  const double t" << x << " = "
-                       << opExpr(nd, nd.a >= 0 ? proRef(nd.a) : "", nd.b >= 0 ? proRef(nd.b) : "",
-                                 nd.c >= 0 ? proRef(nd.c) : "", false)
-                       << ";\n";
-                if (hslot[x] >= 0) hp << "  C[" << hslot[x] << "] = " << proRef((int)x) << ";\n";
-            }
+            std::ostringstream hc;
+            std::vector<ProItem> hitems;
+            for (size_t x = 0; x < n; ++x)
+                if (hslot[x] >= 0) hitems.push_back({hslot[x], (int)x, ""});
             auto ref = [&](int x) -> std::string {
                 const auto& nd = N[x];
                 if (nd.op == dag::Const) return num(nd.v);
@@ -1461,9 +1479,7 @@ std::string Gen::emit()
             tab("d2_th1", d1);
             tab("hrow_der", rder);
             tab("hrow_d2", rd2);
-            hh << "__device__ __forceinline__ void hs_prologue(const double* __restrict__ th, double* __restrict__ C)\n{\n"
-                  "  (void)th; (void)C;\n"
-               << hp.str() << "}\n"
+            hh << prologueText("hs_prologue", "M_NHPRO", hitems)
                << "template <class S>\n__device__ __forceinline__ void hs_columns(const double* __restrict__ ev,\n"
                   "    const double* __restrict__ C, S& s)\n{\n  (void)ev; (void)C;\n"
                << hc.str() << "}\n";

@@ -23,6 +23,7 @@ struct KinSlot {
 };
 
 struct GeneratedModel {
+    std::string id;              // identity of the generated code (hash of the headers below)
     std::string header;          // model.cuh text
     std::string dual_header;     // model_dual.cuh text: the lineshapes in dual numbers (Hessian)
     // model_hess.cuh text: the lineshapes with their first and second theta

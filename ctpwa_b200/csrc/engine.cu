@@ -487,25 +487,6 @@ __global__ void ct_prepare_kernel(const double* __restrict__ params, const int* 
 }
 
 // one block per job of a multi-job evaluation: ct_prepare_kernel's work
-struct PrepareArgs {
-    const double* params;
-    const int* chain;
-    const double* ratio;
-    int nA, nc;
-    double* v;
-    int* err;
-};
-__global__ void ct_prepare_multi_kernel(const PrepareArgs* __restrict__ ps)
-{
-    const PrepareArgs& P = ps[blockIdx.x];
-    if (threadIdx.x == 0 && P.err) *P.err = 0;
-    for (int a = threadIdx.x; a < P.nA; a += blockDim.x) {
-        const int c = P.chain[a];
-        P.v[2 * a] = P.params[c] * P.ratio[a];
-        P.v[2 * a + 1] = P.params[P.nc + c] * P.ratio[a];
-    }
-}
-
 struct FinalizeArgs {
     const double* partials;
     int nacc, nA, nc, nT;
@@ -536,36 +517,50 @@ struct FinalizeArgs {
     const double* phsp_row;
 };
 
-// Per-sample sums of the partial rows plus the sample totals (event-sharded
-// evaluation); the same fixed-order reduction as ct_finalize_kernel (each
-// row read by one warp, the warps' sums added in warp order; launched with
-// 1024 threads and [32][nacc] doubles of dynamic shared memory), so a
-// sharded evaluation on one shard reproduces the unsharded sums bit for bit.
-__global__ void __launch_bounds__(1024) ct_rowsum_kernel(const double* __restrict__ partials, int nacc, FinalizeArgs A,
-                                                         double W_phsp, double* __restrict__ out)
+// Sums of the partial rows of the samples [k0, k1): warp w adds rows w,
+// w + nwarp, ... of each sample (every row read by one warp, lanes over its
+// columns: coalesced), then one thread per (sample, column) adds the warps'
+// sums, every fourth together and the four last, so the sums are
+// bit-reproducible. wsum: [k1 - k0][nwarp][nacc] doubles; out: [3][nacc].
+__device__ __forceinline__ void ct_sum_rows(const FinalizeArgs& A, const double* __restrict__ partials, int nacc, int k0,
+                                            int k1, double* wsum, double* out)
 {
-    extern __shared__ double wsum[];  // [nwarp][nacc]
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int k = 0; k < 3; ++k) {
-        for (int j0 = 0; j0 < nacc; j0 += 32) {
-            const int j = j0 + lane;
-            if (j >= nacc) continue;
+    for (int k = k0; k < k1; ++k)
+        for (int j = lane; j < nacc; j += 32) {
             double s = 0.0;
             if (A.has[k]) {
                 const double* rows = partials + (long long)A.cta[k][0] * nacc + j;
 #pragma unroll 4
                 for (int b = warp; b < A.cta[k][1]; b += nwarp) s += rows[(long long)b * nacc];
             }
-            wsum[warp * nacc + j] = s;
+            wsum[((k - k0) * nwarp + warp) * nacc + j] = s;
         }
-        __syncthreads();
-        for (int j = threadIdx.x; j < nacc; j += blockDim.x) {
-            double s = 0.0;
-            for (int w = 0; w < nwarp; ++w) s += wsum[w * nacc + j];
-            out[k * nacc + j] = s;
-        }
-        __syncthreads();
+    __syncthreads();
+    for (int i = threadIdx.x; i < (k1 - k0) * nacc; i += blockDim.x) {
+        const double* w = wsum + (long long)(i / nacc) * nwarp * nacc + i % nacc;
+        double s[4] = {0.0, 0.0, 0.0, 0.0};
+        for (int r = 0; r < nwarp; r += 4)
+#pragma unroll
+            for (int q = 0; q < 4; ++q) s[q] += w[(long long)(r + q) * nacc];
+        out[k0 * nacc + i] = (s[0] + s[1]) + (s[2] + s[3]);
     }
+    __syncthreads();
+}
+// rows of doubles of wsum: all three samples at once (their loads in flight
+// together: the finalize of 296 rows 8.5 -> TODO us) while they fit, else one by one
+__host__ __device__ __forceinline__ int ct_sum_samples(int nacc) { return nacc <= 200 ? 3 : 1; }
+
+// Per-sample sums of the partial rows plus the sample totals (event-sharded
+// evaluation); the same reduction as ct_finalize_kernel (launched with 1024
+// threads and [ct_sum_samples][32][nacc] doubles of dynamic shared memory), so
+// a sharded evaluation on one shard reproduces the unsharded sums bit for bit.
+__global__ void __launch_bounds__(1024) ct_rowsum_kernel(const double* __restrict__ partials, int nacc, FinalizeArgs A,
+                                                         double W_phsp, double* __restrict__ out)
+{
+    extern __shared__ double wsum[];
+    const int step = ct_sum_samples(nacc);
+    for (int k = 0; k < 3; k += step) ct_sum_rows(A, partials, nacc, k, k + step, wsum, out);
     if (threadIdx.x == 0) {
         out[3 * nacc + 0] = A.n_phsp;
         out[3 * nacc + 1] = W_phsp;
@@ -583,7 +578,7 @@ __device__ __forceinline__ void ct_finalize_body(const FinalizeArgs& A)
     // serial assembly staged by all threads (thread 0 reads no global
     // memory): couplings [2 nA], parameters [2 nc + nT], coupling chain
     // [nA], Gaussian constraints [3 ngauss]; then the per-warp sums of the
-    // row reduction [32][nacc] (ct_finalize_shm)
+    // row reduction (ct_sum_rows, ct_finalize_shm)
     extern __shared__ double sh[];
     double* sums = sh;
     double* sv = sh + 3 * A.nacc + 2 * A.nA + 8;
@@ -598,9 +593,6 @@ __device__ __forceinline__ void ct_finalize_body(const FinalizeArgs& A)
         sg[3 * i + 1] = A.gauss_ms[2 * i];
         sg[3 * i + 2] = A.gauss_ms[2 * i + 1];
     }
-    // one warp per (sample, column): lanes stride over the CTA rows, then a
-    // fixed-order shuffle tree, so the sums are bit-reproducible
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     double n_phsp = A.n_phsp, W_data = A.W_data, W_bkg = A.W_bkg, gv_phsp_scale = 1.0;
     if (A.sums) {
         for (int i = threadIdx.x; i < 3 * A.nacc; i += blockDim.x) sums[i] = A.sums[i];
@@ -610,35 +602,11 @@ __device__ __forceinline__ void ct_finalize_body(const FinalizeArgs& A)
         W_data = A.sums[3 * A.nacc + 2];
         W_bkg = A.sums[3 * A.nacc + 3];
     } else {
-        // per sample: warp w sums rows w, w + nwarp, ... of the sample's CTA
-        // rows (each row read by one warp, lanes over its columns:
-        // coalesced), then one thread per column adds the warps' sums in
-        // warp order, so the sums are bit-reproducible
-        double* wsum = sg + 3 * A.ngauss;  // [nwarp][nacc]
-        for (int k = 0; k < 3; ++k) {
-            if (k == 0 && A.phsp_row) {
-                for (int j = threadIdx.x; j < A.nacc; j += blockDim.x) sums[j] = A.phsp_row[j];
-                continue;
-            }
-            for (int j0 = 0; j0 < A.nacc; j0 += 32) {
-                const int j = j0 + lane;
-                if (j >= A.nacc) continue;
-                double s = 0.0;
-                if (A.has[k]) {
-                    const double* rows = A.partials + (long long)A.cta[k][0] * A.nacc + j;
-#pragma unroll 4
-                    for (int b = warp; b < A.cta[k][1]; b += nwarp) s += rows[(long long)b * A.nacc];
-                }
-                wsum[warp * A.nacc + j] = s;
-            }
-            __syncthreads();
-            for (int j = threadIdx.x; j < A.nacc; j += blockDim.x) {
-                double s = 0.0;
-                for (int w = 0; w < nwarp; ++w) s += wsum[w * A.nacc + j];
-                sums[k * A.nacc + j] = s;
-            }
-            __syncthreads();
-        }
+        double* wsum = sg + 3 * A.ngauss;
+        const int step = ct_sum_samples(A.nacc), k0 = A.phsp_row ? 1 : 0;
+        if (A.phsp_row)
+            for (int j = threadIdx.x; j < A.nacc; j += blockDim.x) sums[j] = A.phsp_row[j];
+        for (int k = k0; k < 3; k += step) ct_sum_rows(A, A.partials, A.nacc, k, min(k + step, 3), wsum, sums);
     }
     __syncthreads();
     // loss and gradient assembly, spread over threads: thread 0 the loss,
@@ -733,7 +701,7 @@ __global__ void __launch_bounds__(1024) ct_finalize_kernel(FinalizeArgs A) { ct_
 size_t ct_finalize_shm(const FinalizeArgs& f)
 {
     return sizeof(double) * (3 * (size_t)f.nacc + 4 * (size_t)f.nA + 8 + 2 * (size_t)f.nc + f.nT + f.nA +
-                             3 * (size_t)f.ngauss + 32 * (size_t)f.nacc);
+                             3 * (size_t)f.ngauss + 32 * (size_t)ct_sum_samples(f.nacc) * f.nacc);
 }
 
 // one CTA per job of a multi-job evaluation (all jobs of one model: same shared-memory size)
@@ -760,6 +728,8 @@ std::string readFile(const std::string& p)
 // configuration text, its chain-filter patterns and its lineshape tables:
 // handles built from the same ones (a serving loop creates several per model)
 // share one generated model.
+uint64_t fnv1a(const std::string& s);
+
 GeneratedModel cachedGenerate(const Model& m, const std::string& config_path)
 {
     std::string key = readFile(config_path);
@@ -776,7 +746,15 @@ GeneratedModel cachedGenerate(const Model& m, const std::string& config_path)
         auto it = cache.find(key);
         if (it != cache.end()) return *it->second;
     }
-    auto g = std::make_shared<const GeneratedModel>(generateModel(m));
+    auto fresh = std::make_shared<GeneratedModel>(generateModel(m));
+    {
+        char id[64];
+        const std::string all = fresh->header + fresh->dual_header + fresh->hess_header;
+        std::snprintf(id, sizeof id, "%016llx%016llx", (unsigned long long)fnv1a(all),
+                      (unsigned long long)std::hash<std::string>{}(all));
+        fresh->id = id;
+    }
+    std::shared_ptr<const GeneratedModel> g = fresh;
     std::lock_guard<std::mutex> lk(mu);
     if (cache.size() >= 32) cache.clear();
     cache.emplace(key, g);
@@ -823,6 +801,51 @@ std::string cacheDir()
 }
 
 }  // namespace
+
+// Loaded kernel modules between handles. A handle needs modules of its own
+// (the per-call constant block is a module global, and handles on different
+// streams must not share it), but loading one costs 1-1.5 ms, most of a small
+// toy job's set-up: a handle that goes returns its modules here, and the next
+// handle of the same generated code, options and device takes them over
+// (its first call rewrites the constant block). At most kMax modules wait;
+// beyond that the one idle longest is unloaded.
+class ModulePool {
+public:
+    static constexpr size_t kMax = 16;
+    static ModulePool& get()
+    {
+        static ModulePool* p = new ModulePool;  // outlives every handle; the driver unloads at exit
+        return *p;
+    }
+    cudaLibrary_t take(const std::string& key)
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        for (size_t i = idle_.size(); i-- > 0;)
+            if (idle_[i].first == key) {
+                cudaLibrary_t lib = idle_[i].second;
+                idle_.erase(idle_.begin() + (long)i);
+                return lib;
+            }
+        return nullptr;
+    }
+    void give(const std::string& key, cudaLibrary_t lib)
+    {
+        cudaLibrary_t drop = nullptr;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            idle_.emplace_back(key, lib);
+            if (idle_.size() > kMax) {
+                drop = idle_.front().second;
+                idle_.erase(idle_.begin());
+            }
+        }
+        if (drop) cudaLibraryUnload(drop);
+    }
+
+private:
+    std::mutex mu_;
+    std::vector<std::pair<std::string, cudaLibrary_t>> idle_;  // oldest first
+};
 
 // The library's device-memory pool of one device (created on first use,
 // kept for the process): freed blocks stay in the pool for later handles.
@@ -1082,12 +1105,7 @@ Engine::~Engine()
         cudaStreamSynchronize(mem_stream_);
         cudaStreamDestroy(mem_stream_);
     }
-    if (hvp_lib_) cudaLibraryUnload((cudaLibrary_t)hvp_lib_);
-    if (hess_lib_) cudaLibraryUnload((cudaLibrary_t)hess_lib_);
-    if (gram_lib_) cudaLibraryUnload((cudaLibrary_t)gram_lib_);
-    if (gram_hess_lib_) cudaLibraryUnload((cudaLibrary_t)gram_hess_lib_);
-    if (norm_lib_) cudaLibraryUnload((cudaLibrary_t)norm_lib_);
-    if (lib_) cudaLibraryUnload((cudaLibrary_t)lib_);
+    for (auto& m : modules_) ModulePool::get().give(m.first, (cudaLibrary_t)m.second);
 }
 
 void Engine::loadSamples()
@@ -2127,16 +2145,41 @@ bool angularInterpreted()
     return e && *e && *e != '0';
 }
 
+std::string shapeKey(const FusedShape& sh)
+{
+    std::string k;
+    for (int i = 0; i < 2; ++i)
+        for (int v : {sh.block[i], sh.minb[i], sh.acc[i], sh.stage[i]}) k += std::to_string(v) + " ";
+    return k;
+}
+
+// This handle's module of the given kind: one another handle has left, or the
+// cubin loaded anew. It goes back when the handle is destroyed.
+template <class Cubin>
+void* Engine::takeModule(const std::string& kind, const Cubin& cubin)
+{
+    const std::string key = gen_.id + " " + std::to_string(opt_.device) + " " + kind;
+    cudaLibrary_t lib = ModulePool::get().take(key);
+    if (!lib) {
+        const std::string image = cubin();
+        CT_CUDA(cudaLibraryLoadData(&lib, image.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
+    } else if (kind.rfind("fused", 0) == 0) {
+        jit_cache_hit_ = true;
+    }
+    modules_.emplace_back(key, (void*)lib);
+    return (void*)lib;
+}
+
 void Engine::compileKernel()
 {
     auto t0 = std::chrono::steady_clock::now();
-    std::string cubin = jitCubin(gen_, &jit_cache_hit_);
-    cudaLibrary_t lib;
-    CT_CUDA(cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-    lib_ = (void*)lib;
+    cudaLibrary_t lib = (cudaLibrary_t)takeModule("fused " + shapeKey(shape_), [&] { return jitCubin(gen_, &jit_cache_hit_); });
     cudaKernel_t k64, kmx, kin, kpro;
     CT_CUDA(cudaLibraryGetKernel(&kpro, lib, "ct_prologue"));
     k_pro_ = (void*)kpro;
+    cudaKernel_t kproh;
+    CT_CUDA(cudaLibraryGetKernel(&kproh, lib, "ct_prologue_host"));
+    k_pro_host_ = (void*)kproh;
     cudaKernel_t kevc;
     CT_CUDA(cudaLibraryGetKernel(&kevc, lib, "ct_event_cache"));
     k_evc_ = (void*)kevc;
@@ -2174,7 +2217,7 @@ void Engine::compileKernel()
                 CT_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, shape_.dsmem[pr]));
     k_int_ = (void*)kin;
     {
-        std::string key = gen_.header;
+        std::string key = gen_.id;
         for (int pr = 0; pr < 2; ++pr)
             key += "|" + std::to_string(shape_.block[pr]) + "," + std::to_string(shape_.minb[pr]) + "," +
                    std::to_string(shape_.dsmem[pr]);
@@ -2259,15 +2302,45 @@ struct CtArgsH {
     int pad2;
     int* err;
     void* kblock;
+    double* params;
+    const int* chain;
+    const double* ratio;
+    double* vout;
+    int* err_reset;
+    int nc;
+    int pad3;
 };
+constexpr int kPrologueBlock = 512;   // CT_PRO_BLOCK
 
-void Engine::nllGrad(const double* d_params, double* d_nll, double* d_grad, int precision, cudaStream_t stream)
+// the prologue's fields of one call's arguments (a.v is set)
+void Engine::prologueArgs(CtArgsH& a, const double* d_params, int* err_reset) const
+{
+    a.theta = d_params + 2 * model_.nVector();
+    a.params = const_cast<double*>(d_params);
+    a.chain = d_amp_chain_;
+    a.ratio = d_ratio_;
+    a.vout = const_cast<double*>(a.v);
+    a.err_reset = err_reset;
+    a.nc = model_.nVector();
+}
+
+// The prologue of one call. host_params: the parameters in host memory; they
+// travel as kernel arguments and are stored to d_params (nParams() <=
+// kHostParamsMax).
+void Engine::launchPrologue(CtArgsH& a, const double* d_params, int* err_reset, cudaStream_t stream,
+                            const double* host_params)
+{
+    prologueArgs(a, d_params, err_reset);
+    void* args[] = {&a, const_cast<double*>(host_params)};
+    CT_CUDA(cudaLaunchKernel(host_params ? k_pro_host_ : k_pro_, dim3(1), dim3(kPrologueBlock), args, 0, stream));
+}
+
+void Engine::nllGrad(const double* d_params, double* d_nll, double* d_grad, int precision, cudaStream_t stream,
+                     const double* host_params)
 {
     const CtaLayout& lay = lay_[precision == kMixed ? 1 : 0];
     const Model& m = model_;
     int nA = m.nAmp(), nc = m.nVector(), nT = m.nTheta();
-    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, nc, d_v_, d_err_);
-    CT_CUDA(cudaGetLastError());
     CtArgsH a;
     std::memset(&a, 0, sizeof(a));
     int ns = 0;
@@ -2294,8 +2367,8 @@ void Engine::nllGrad(const double* d_params, double* d_nll, double* d_grad, int 
     a.err = d_err_;
     a.kblock = d_kblock_;
     if (precision == kMixed && !samples_[0].slamp32) throw std::runtime_error("mixed-precision tables were not built");
+    launchPrologue(a, d_params, d_err_, stream, host_params);
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(k_sym_, d_kblock_, k_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
     const size_t slot = ev_begin_.empty() ? 0 : (size_t)(ev_count_ % (long long)ev_begin_.size());
     if (!ev_begin_.empty()) CT_CUDA(cudaEventRecord(ev_begin_[slot], stream));
@@ -2370,9 +2443,9 @@ void Engine::nllGradMulti(const std::vector<Engine*>& es, const std::vector<cons
         if (precision == kMixed && !e->samples_[0].slamp32)
             throw std::runtime_error("mixed-precision tables were not built");
     }
-    // staging: [CtArgsH x nj][PrepareArgs x nj][FinalizeArgs x nj][cta_off x (nj + 1)]
+    // staging: [CtArgsH x nj][FinalizeArgs x nj][cta_off x (nj + 1)]
     auto up = [](size_t x) { return (x + 255) / 256 * 256; };
-    const size_t o_args = 0, o_prep = up(sizeof(CtArgsH) * nj), o_fin = o_prep + up(sizeof(PrepareArgs) * nj),
+    const size_t o_args = 0, o_fin = up(sizeof(CtArgsH) * nj),
                  o_off = o_fin + up(sizeof(FinalizeArgs) * nj), bytes = o_off + up(sizeof(int) * (nj + 1));
     if (!sc.copied) CT_CUDA(cudaEventCreateWithFlags(&sc.copied, cudaEventDisableTiming));
     CT_CUDA(cudaEventSynchronize(sc.copied));  // the previous call's copy has left the host buffer
@@ -2388,7 +2461,6 @@ void Engine::nllGradMulti(const std::vector<Engine*>& es, const std::vector<cons
     unsigned char* hb = (unsigned char*)sc.host;
     unsigned char* db = (unsigned char*)sc.dev;
     CtArgsH* ha = (CtArgsH*)(hb + o_args);
-    PrepareArgs* hp = (PrepareArgs*)(hb + o_prep);
     FinalizeArgs* hf = (FinalizeArgs*)(hb + o_fin);
     int* hoff = (int*)(hb + o_off);
     int total = 0, shm_max = 0;
@@ -2417,14 +2489,13 @@ void Engine::nllGradMulti(const std::vector<Engine*>& es, const std::vector<cons
             smp.vw_scale = 1.0 / (e->samples_[0].wsum > 0 ? e->samples_[0].wsum : 1.0);
         }
         a.nsamp = ns;
-        a.theta = d_params[j] + 2 * nc;
         a.v = e->d_v_;
         a.partials = e->d_partials_;
         a.consts = e->d_consts_;
         a.err = e->d_err_;
         a.kblock = e->d_kblock_;
         a.cta_base = -total;
-        hp[j] = PrepareArgs{d_params[j], e->d_amp_chain_, e->d_ratio_, nA, nc, e->d_v_, e->d_err_};
+        e->prologueArgs(a, d_params[j], e->d_err_);
         FinalizeArgs& f = hf[j];
         std::memset(&f, 0, sizeof(f));
         f.partials = e->d_partials_;
@@ -2457,11 +2528,9 @@ void Engine::nllGradMulti(const std::vector<Engine*>& es, const std::vector<cons
     hoff[nj] = total;
     CT_CUDA(cudaMemcpyAsync(db, hb, bytes, cudaMemcpyHostToDevice, stream));
     CT_CUDA(cudaEventRecord(sc.copied, stream));
-    ct_prepare_multi_kernel<<<nj, 128, 0, stream>>>((const PrepareArgs*)(db + o_prep));
-    CT_CUDA(cudaGetLastError());
     const CtArgsH* dargs = (const CtArgsH*)(db + o_args);
     void* pargs[] = {&dargs};
-    CT_CUDA(cudaLaunchKernel(e0->k_pro_multi_, dim3(nj), dim3(64), pargs, 0, stream));
+    CT_CUDA(cudaLaunchKernel(e0->k_pro_multi_, dim3(nj), dim3(kPrologueBlock), pargs, 0, stream));
     const int* doff = (const int*)(db + o_off);
     int njobs = nj;
     void* fargs[] = {&dargs, &doff, &njobs};
@@ -2543,8 +2612,6 @@ void Engine::nllGradStatic(const double* d_params, double* d_nll, double* d_grad
     double* s_partials = base + off_p;
     double* s_parts = base + off_parts;
 
-    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, nc, s_v, (int*)(base + off_err));
-    CT_CUDA(cudaGetLastError());
     CtArgsH a;
     std::memset(&a, 0, sizeof(a));
     int ns = 0;
@@ -2571,8 +2638,8 @@ void Engine::nllGradStatic(const double* d_params, double* d_nll, double* d_grad
     a.err = (int*)(base + off_err);
     a.kblock = base + off_k;
     if (precision == kMixed && !samples_[0].slamp32) throw std::runtime_error("mixed-precision tables were not built");
+    launchPrologue(a, d_params, (int*)(base + off_err), stream);
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(k_sym_, base + off_k, k_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
     a.cta_base = 0;
     CT_CUDA(cudaLaunchKernel(precision == kMixed ? k_mixed_ : k_f64_, dim3(lay.grid), dim3(shape_.block[precision == kMixed]),
@@ -2615,8 +2682,6 @@ void Engine::shardSums(const double* d_params, int precision, double* d_sums, cu
     const Model& m = model_;
     const int nA = m.nAmp(), nc = m.nVector(), nT = m.nTheta();
     const int nacc = 2 + 2 * nA + nT;
-    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, nc, d_v_, d_err_);
-    CT_CUDA(cudaGetLastError());
     CtArgsH a;
     std::memset(&a, 0, sizeof(a));
     int ns = 0;
@@ -2643,8 +2708,8 @@ void Engine::shardSums(const double* d_params, int precision, double* d_sums, cu
     a.err = d_err_;
     a.kblock = d_kblock_;
     if (precision == kMixed && !samples_[0].slamp32) throw std::runtime_error("mixed-precision tables were not built");
+    launchPrologue(a, d_params, d_err_, stream);
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(k_sym_, d_kblock_, k_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
     a.cta_base = 0;
     CT_CUDA(cudaLaunchKernel(precision == kMixed ? k_mixed_ : k_f64_, dim3(lay.grid), dim3(shape_.block[precision == kMixed]),
@@ -2659,7 +2724,7 @@ void Engine::shardSums(const double* d_params, int precision, double* d_sums, cu
     f.n_phsp = (double)samples_[0].n;
     f.W_data = samples_[1].wsum;
     f.W_bkg = has_bkg_ ? samples_[2].wsum : 0.0;
-    ct_rowsum_kernel<<<1, 1024, sizeof(double) * 32 * (size_t)nacc, stream>>>(d_partials_, nacc, f, samples_[0].wsum,
+    ct_rowsum_kernel<<<1, 1024, sizeof(double) * 32 * (size_t)ct_sum_samples(nacc) * nacc, stream>>>(d_partials_, nacc, f, samples_[0].wsum,
                                                                                d_sums);
     CT_CUDA(cudaGetLastError());
 }
@@ -2964,11 +3029,7 @@ void Engine::compileHvp()
     hvpBuffers();
     if (k_hvp_) return;
     RelaxedCapture relaxed;
-    bool hit = false;
-    std::string cubin = jitHvpCubin(gen_, paired_[0], &hit);
-    cudaLibrary_t lib;
-    CT_CUDA(cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-    hvp_lib_ = (void*)lib;
+    cudaLibrary_t lib = (cudaLibrary_t)takeModule(paired_[0] ? "hvp paired" : "hvp", [&] { return jitHvpCubin(gen_, paired_[0], nullptr); });
     cudaKernel_t kp, kh;
     CT_CUDA(cudaLibraryGetKernel(&kp, lib, "ct_hvp_prologue"));
     CT_CUDA(cudaLibraryGetKernel(&kh, lib, "ct_hvp_f64"));
@@ -2996,11 +3057,7 @@ void Engine::compileHess()
     if (k_hess_) return;
     RelaxedCapture relaxed;
     const HessShape h = hessShape(gen_);
-    bool hit = false;
-    std::string cubin = jitHessCubin(gen_, paired_[0], &hit);
-    cudaLibrary_t lib;
-    CT_CUDA(cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-    hess_lib_ = (void*)lib;
+    cudaLibrary_t lib = (cudaLibrary_t)takeModule(paired_[0] ? "hess paired" : "hess", [&] { return jitHessCubin(gen_, paired_[0], nullptr); });
     cudaKernel_t kp, kh, kr, kc;
     CT_CUDA(cudaLibraryGetKernel(&kp, lib, "ct_hess_prologue"));
     CT_CUDA(cudaLibraryGetKernel(&kh, lib, "ct_hess_f64"));
@@ -3086,7 +3143,7 @@ void Engine::hessSums(const double* d_params, const double* d_dirs, int ndir, do
     a.img = d_hess_img_;
     a.rows = d_hess_rows_;
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_hess_pro_, dim3(1), dim3(32), args, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_hess_pro_, dim3(1), dim3(512), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(hess_sym_, d_hess_img_, hess_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
     if (a.nsamp > 0)
         CT_CUDA(cudaLaunchKernel(k_hess_, dim3(hess_grid_), dim3(32 * h.warps), args, (size_t)h.dsmem, stream));
@@ -3255,11 +3312,7 @@ void Engine::compileGram()
         throw std::length_error("the tensor-core Gram supports npol * 2 * nA <= 128; this model has " +
                                 std::to_string(rows));
     if (!samples_[0].slamp32) throw std::runtime_error("the Gram needs the mixed-precision tables");
-    bool hit = false;
-    std::string cubin = jitGramCubin(gen_, paired_[1], &hit);
-    cudaLibrary_t lib;
-    CT_CUDA(cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-    gram_lib_ = (void*)lib;
+    cudaLibrary_t lib = (cudaLibrary_t)takeModule(paired_[1] ? "gram paired" : "gram", [&] { return jitGramCubin(gen_, paired_[1], nullptr); });
     cudaKernel_t kg, kf;
     CT_CUDA(cudaLibraryGetKernel(&kg, lib, "ct_gram"));
     CT_CUDA(cudaLibraryGetKernel(&kf, lib, "ct_gram_finalize"));
@@ -3295,11 +3348,7 @@ void Engine::compileGramHess()
         throw std::length_error("the Gram-based Hessian supports (npol + 1) * 2 * nA <= 128; this model has " +
                                 std::to_string(rows));
     if (!samples_[0].slamp32) throw std::runtime_error("the Gram needs the mixed-precision tables");
-    bool hit = false;
-    std::string cubin = jitGramCubin(gen_, paired_[1], &hit, true);
-    cudaLibrary_t lib;
-    CT_CUDA(cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-    gram_hess_lib_ = (void*)lib;
+    cudaLibrary_t lib = (cudaLibrary_t)takeModule(paired_[1] ? "gram-hess paired" : "gram-hess", [&] { return jitGramCubin(gen_, paired_[1], nullptr, true); });
     cudaKernel_t kg, kf;
     CT_CUDA(cudaLibraryGetKernel(&kg, lib, "ct_gram"));
     CT_CUDA(cudaLibraryGetKernel(&kf, lib, "ct_gram_hess_finalize"));
@@ -3521,11 +3570,7 @@ void Engine::compileNorm()
     if (groups > 128 || nt + nd > 256 || (size_t)(2 * nt + nd) * nt * 16 > 40000)
         throw std::length_error("the normalisation cache supports models with up to 256 lineshape terms and "
                                 "derivative entries and (2 terms + entries) x terms <= 2500");
-    bool hit = false;
-    std::string cubin = jitNormCubin(gen_, &hit);
-    cudaLibrary_t lib;
-    CT_CUDA(cudaLibraryLoadData(&lib, cubin.data(), nullptr, nullptr, 0, nullptr, nullptr, 0));
-    norm_lib_ = (void*)lib;
+    cudaLibrary_t lib = (cudaLibrary_t)takeModule("norm", [&] { return jitNormCubin(gen_, nullptr); });
     cudaKernel_t kb, kr, kw;
     CT_CUDA(cudaLibraryGetKernel(&kb, lib, "ct_norm_build"));
     CT_CUDA(cudaLibraryGetKernel(&kr, lib, "ct_norm_reduce"));
@@ -3559,15 +3604,12 @@ double Engine::normCacheBuild(const double* d_params, cudaStream_t stream)
     const int nA = m.nAmp(), nc = m.nVector(), nT = m.nTheta();
     norm_valid_ = false;
     // the parameter-only subexpressions at this theta
-    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, nc, d_v_, nullptr);
-    CT_CUDA(cudaGetLastError());
     CtArgsH pa;
     std::memset(&pa, 0, sizeof(pa));
     pa.theta = d_params + 2 * nc;
     pa.v = d_v_;
     pa.consts = d_consts_;
-    void* pargs[] = {&pa};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), pargs, 0, stream));
+    launchPrologue(pa, d_params, nullptr, stream);
     const DeviceSample& d = samples_[0];
     CtNormArgsH a;
     std::memset(&a, 0, sizeof(a));
@@ -3590,7 +3632,7 @@ double Engine::normCacheBuild(const double* d_params, cudaStream_t stream)
     double* part = d_npart_;
     double* mat = d_nmat_;
     void* rargs[] = {&part, &rows, &ne, &mat};
-    CT_CUDA(cudaLaunchKernel(k_norm_red_, dim3(1), dim3(256), rargs, 0, stream));
+    CT_CUDA(cudaLaunchKernel(k_norm_red_, dim3((2 * ne + 31) / 32), dim3(256), rargs, 0, stream));
     if (nT > 0)
         CT_CUDA(cudaMemcpyAsync(d_ntheta_, d_params + 2 * nc, sizeof(double) * nT, cudaMemcpyDeviceToDevice, stream));
     norm_theta_.assign(nT, 0.0);
@@ -3616,14 +3658,13 @@ bool Engine::normCacheMatches(const double* params) const
 // The evaluation at the cached resonance parameters: the fused pass over the
 // data and background samples (their own one-wave layout), the phase-space
 // row from the matrices, the usual finalize.
-void Engine::nllGradCached(const double* d_params, double* d_nll, double* d_grad, int precision, cudaStream_t stream)
+void Engine::nllGradCached(const double* d_params, double* d_nll, double* d_grad, int precision, cudaStream_t stream,
+                           const double* host_params)
 {
     if (!norm_valid_) throw std::runtime_error("no normalisation cache: build it first");
     const CtaLayout& lay = lay_data_[precision == kMixed ? 1 : 0];
     const Model& m = model_;
     const int nA = m.nAmp(), nc = m.nVector(), nT = m.nTheta();
-    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, nc, d_v_, d_err_);
-    CT_CUDA(cudaGetLastError());
     CtArgsH a;
     std::memset(&a, 0, sizeof(a));
     int ns = 0;
@@ -3650,8 +3691,8 @@ void Engine::nllGradCached(const double* d_params, double* d_nll, double* d_grad
     a.err = d_err_;
     a.kblock = d_kblock_;
     if (precision == kMixed && !samples_[1].slamp32) throw std::runtime_error("mixed-precision tables were not built");
+    launchPrologue(a, d_params, d_err_, stream, host_params);
     void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(k_sym_, d_kblock_, k_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
     a.cta_base = 0;
     if (ns > 0)
@@ -3718,8 +3759,6 @@ void Engine::gram(const double* d_params, double* d_out, cudaStream_t stream)
     const Model& m = model_;
     const int nA = m.nAmp(), nc = m.nVector();
     // this call's couplings and parameter-only constants (the constant-bank image)
-    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, nc, d_v_, d_err_);
-    CT_CUDA(cudaGetLastError());
     CtArgsH a;
     std::memset(&a, 0, sizeof(a));
     a.theta = d_params + 2 * nc;
@@ -3727,8 +3766,7 @@ void Engine::gram(const double* d_params, double* d_out, cudaStream_t stream)
     a.consts = d_consts_;
     a.err = d_err_;
     a.kblock = d_kblock_;
-    void* args[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), args, 0, stream));
+    launchPrologue(a, d_params, d_err_, stream);
     const DeviceSample& d = samples_[0];
     CtGramArgsH g;
     std::memset(&g, 0, sizeof(g));
@@ -3838,8 +3876,6 @@ void Engine::partialIntegrals(const double* d_params, int kind, double* d_out, c
     const Model& m = model_;
     const int nA = m.nAmp(), nc = m.nVector(), nb = nBlocks();
     const DeviceSample& d = samples_[kind];
-    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, nc, d_v_, nullptr);
-    CT_CUDA(cudaGetLastError());
     CtArgsH a;
     std::memset(&a, 0, sizeof(a));
     a.s[0].slamp = d.slamp64;
@@ -3855,8 +3891,7 @@ void Engine::partialIntegrals(const double* d_params, int kind, double* d_out, c
     a.partials = d_partials_;
     a.consts = d_consts_;
     a.err = d_err_;
-    void* pargs[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), pargs, 0, stream));
+    launchPrologue(a, d_params, nullptr, stream);
     // rows of nb sums in the partials table (nacc >= nA >= nb columns per row available)
     const int nacc = 2 + 2 * nA + m.nTheta();
     const long long cap_rows = (long long)grid_max_ * nacc / std::max(1, nb);
@@ -3876,8 +3911,6 @@ void Engine::exportWeights(const double* d_params, const std::vector<int>& mask,
     const int npair = nb * (nb + 1) / 2;
     if (!mask.empty() && (int)mask.size() != nb) throw std::runtime_error("export: wave mask must have one entry per block");
     const DeviceSample& d = samples_[0];
-    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, nc, d_v_, nullptr);
-    CT_CUDA(cudaGetLastError());
     CtArgsH a;
     std::memset(&a, 0, sizeof(a));
     a.s[0].slamp = d.slamp64;
@@ -3892,8 +3925,7 @@ void Engine::exportWeights(const double* d_params, const std::vector<int>& mask,
     a.partials = d_partials_;
     a.consts = d_consts_;
     a.err = d_err_;
-    void* pargs[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), pargs, 0, stream));
+    launchPrologue(a, d_params, nullptr, stream);
     const int* dmask = nullptr;
     if (!mask.empty()) {
         CT_CUDA(cudaMemcpyAsync(d_mask_, mask.data(), sizeof(int) * nb, cudaMemcpyHostToDevice, stream));
@@ -3914,8 +3946,6 @@ void Engine::intensity(const double* d_params, int kind, double* d_out, cudaStre
     if (kind < 0 || kind > 2 || samples_[kind].n == 0) throw std::runtime_error("intensity: empty or unknown sample");
     const Model& m = model_;
     int nA = m.nAmp(), nc = m.nVector();
-    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, nc, d_v_, nullptr);
-    CT_CUDA(cudaGetLastError());
     CtArgsH a;
     std::memset(&a, 0, sizeof(a));
     const DeviceSample& d = samples_[kind];
@@ -3931,8 +3961,7 @@ void Engine::intensity(const double* d_params, int kind, double* d_out, cudaStre
     a.partials = d_partials_;
     a.consts = d_consts_;
     a.err = d_err_;
-    void* pargs[] = {&a};
-    CT_CUDA(cudaLaunchKernel(k_pro_, dim3(1), dim3(64), pargs, 0, stream));
+    launchPrologue(a, d_params, nullptr, stream);
     void* args[] = {&a, &d_out};
     int grid = (int)std::min<long long>((d.n + 255) / 256, 148LL * 16);
     CT_CUDA(cudaLaunchKernel(k_int_, dim3(grid), dim3(256), args, 0, stream));

@@ -91,6 +91,8 @@ void phaseSpace(double M, const double* masses, long long n, unsigned long long 
 // Stream-ordered, no host synchronisation (csrc/linalg.cu).
 void spdInverse(const double* d_a, int n, double* d_out, int* d_info, cudaStream_t stream);
 
+struct CtArgsH;  // argument block of the fused kernels
+
 class Engine {
 public:
     Engine(const std::string& config_path, const EngineOptions& opt);
@@ -103,7 +105,13 @@ public:
 
     // NLL and gradient in the reference layout [Re p, Im p, theta]; all
     // pointers are device pointers; stream-ordered, no host synchronisation.
-    void nllGrad(const double* d_params, double* d_nll, double* d_grad, int precision, cudaStream_t stream);
+    // host_params: the parameters in host memory (read before the call
+    // returns; at most kHostParamsMax): they travel with the first launch and
+    // d_params is their device copy, written by it. d_nll and d_grad may be
+    // pinned host memory.
+    static constexpr int kHostParamsMax = 400;
+    void nllGrad(const double* d_params, double* d_nll, double* d_grad, int precision, cudaStream_t stream,
+                 const double* host_params = nullptr);
     // The same evaluation with its scratch (couplings, parameter-only
     // constants, per-CTA partial rows, per-sample parts) in one fixed array
     // compiled into the library instead of the handle's buffers; allocates
@@ -145,7 +153,8 @@ public:
     bool normCacheValid() const { return norm_valid_; }
     // true when the cache is valid for the resonance parameters of the host array params
     bool normCacheMatches(const double* params) const;
-    void nllGradCached(const double* d_params, double* d_nll, double* d_grad, int precision, cudaStream_t stream);
+    void nllGradCached(const double* d_params, double* d_nll, double* d_grad, int precision, cudaStream_t stream,
+                       const double* host_params = nullptr);
     static constexpr size_t kStaticScratchBytes = size_t(2) << 20;
     // Event-sharded evaluation: the per-sample sums of this handle's events,
     // [3][nacc] + [n_phsp, W_phsp, W_data, W_bkg] (sumsSize() doubles), ready
@@ -232,7 +241,6 @@ private:
     bool onePassHessian(int ndir) const;
     void hessSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums, double* d_vsums,
                   cudaStream_t stream);
-    void* hess_lib_ = nullptr;
     void* k_hess_pro_ = nullptr;
     void* k_hess_ = nullptr;
     void* k_hess_red_ = nullptr;
@@ -260,8 +268,10 @@ private:
     struct GroupDev;
     std::vector<std::vector<char>> group_desc_;  // AgGroup images per group
 
-    // JIT
-    void* lib_ = nullptr;  // cudaLibrary_t
+    // kernel modules (cudaLibrary_t) with their pool keys
+    std::vector<std::pair<std::string, void*>> modules_;
+    template <class Cubin>
+    void* takeModule(const std::string& kind, const Cubin& cubin);
     void* k_f64_ = nullptr;
     void* k_mixed_ = nullptr;
     void* k_int_ = nullptr;
@@ -269,20 +279,22 @@ private:
     void* k_exp_ = nullptr;
     int* d_mask_ = nullptr;  // [nBlocks] export wave mask
     void* k_pro_ = nullptr;
+    void* k_pro_host_ = nullptr;
+    void prologueArgs(CtArgsH& a, const double* d_params, int* err_reset) const;
+    void launchPrologue(CtArgsH& a, const double* d_params, int* err_reset, cudaStream_t stream,
+                        const double* host_params = nullptr);
     void* k_multi_[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};  // [plain, mixed][paired]
     void* k_pro_multi_ = nullptr;
     const void* image_key_ = nullptr;
     // tensor-core Gram (compiled on the first request)
     void compileGram();
     void compileGramHess();
-    void* gram_hess_lib_ = nullptr;
     void* k_gramh_ = nullptr;
     void* k_gramh_fin_ = nullptr;
     int gramh_grid_ = 0;
     int gramh_dsmem_ = 0;
     double* d_ghpart_ = nullptr;
     double* d_ghout_ = nullptr;
-    void* gram_lib_ = nullptr;
     void* k_gram_ = nullptr;
     void* k_gram_fin_ = nullptr;
     int gram_grid_ = 0;
@@ -291,7 +303,6 @@ private:
     double* d_gpart_ = nullptr;
     // normalisation cache (compiled and allocated on the first build)
     void compileNorm();
-    void* norm_lib_ = nullptr;
     void* k_norm_build_ = nullptr;
     void* k_norm_red_ = nullptr;
     void* k_norm_row_ = nullptr;
@@ -346,7 +357,6 @@ private:
     void layoutCtas(int target, long long tot, int block, CtaLayout& lay, bool no_phsp = false) const;
 
     // Hessian-vector products (compiled and allocated on first use)
-    void* hvp_lib_ = nullptr;  // cudaLibrary_t
     void* k_hvp_pro_ = nullptr;
     void* k_hvp_ = nullptr;
     int hvp_block_ = 128;

@@ -9,7 +9,8 @@
 //       variant, SL combination) of term t: a column is the sum of its terms
 //       (one term, or one per permutation of identical particles)
 //   der_term(k), der_th(k)   term / theta index of derivative entry k
-//   model_prologue(theta, C)   parameter-only subexpressions, once per call
+//   model_prologue(part, theta, C)   parameter-only subexpressions and the
+//       Jacobian of the adjoint constants, once per call, in M_NPRO parts
 //   model_event(kin, o), model_event_mx(o, of, od)   the parameter-independent
 //       per-event values the per-call code reads (frontier), evaluated once
 //       per event by ct_event_cache when a sample is loaded (FP64; the mixed
@@ -22,8 +23,8 @@
 //   model_adjoint(ev, C, sink)   the values alone, then the adjoints of the
 //       M_NADJ parameter-only constants they read (reverse mode);
 //       model_adjoint_f32(...): the values and the derivatives times the seeds
-//   model_jacobian(theta, J), model_theta_sum(j, J, a)   d constants / d theta,
-//       once per call, and the theta gradient sums from the adjoint sums
+//   model_theta_sum(j, J, a)   the theta gradient sums from the adjoint sums
+//       and the Jacobian J
 //
 // Per event e of a sample (phase space, data or background) the kernel forms
 //   A_{a,p} = F_a * SL_{plane(a),p},   S_p = sum_a v_a A_{a,p},   f = sum_p |S_p|^2
@@ -108,6 +109,16 @@ struct CtArgs {
     int pad2;
     int* err;             // set to 1 when a staged copy did not arrive in time
     void* kblock;         // CtConsts image of this call (written by ct_prologue) or nullptr
+    // for the prologue: parameters [Re p, Im p, theta], coupling of each
+    // amplitude column and its ratio, number of couplings, the couplings'
+    // buffer (v) and an error flag to reset (or nullptr)
+    double* params;
+    const int* chain;
+    const double* ratio;
+    double* vout;
+    int* err_reset;
+    int nc;
+    int pad3;
 };
 
 #define CT_NCONST_ALLOC (M_NCONST > 0 ? M_NCONST : 1)
@@ -137,38 +148,66 @@ struct CtConsts {
 };
 __constant__ CtConsts ct_k;
 
-// The parameter-only part of every lineshape and the Jacobian of the adjoint
-// constants (prologue, one thread of a warp each), then the constant-bank
-// image of this call (64 threads).
-__device__ __forceinline__ void ct_prologue_body(const CtArgs& A);
-extern "C" __global__ void ct_prologue(CtArgs A)
+// One call's inputs from its parameters, by one CTA: the couplings
+// v_a = ratio_a p_chain(a), the parameter-only part of every lineshape with
+// the Jacobian of the adjoint constants (one thread of a warp per part: the
+// dependent FP64 chains run side by side, 5.3 -> 2.6 us on three chains of rho), and
+// the constant-bank image. P: the parameters come with the launch and are
+// stored to A.params for the finalize, without a copy ahead of the kernel.
+#define CT_PRO_BLOCK 512
+struct CtHostParams {
+    double p[M_NPAR];
+};
+__device__ __noinline__ void ct_prologue_body(const CtArgs& A, const CtHostParams* P)
 {
-    if (blockIdx.x != 0) return;
-    ct_prologue_body(A);
-}
-// one block per job of a multi-job evaluation
-extern "C" __global__ void ct_prologue_multi(const CtArgs* __restrict__ jobs) { ct_prologue_body(jobs[blockIdx.x]); }
-
-__device__ __forceinline__ void ct_prologue_body(const CtArgs& A)
-{
-    if (threadIdx.x == 0) model_prologue(A.theta, A.consts);
-    if (threadIdx.x == 32) model_jacobian(A.theta, A.consts + M_NCONST);
+    __shared__ double sp[M_NPAR], sc[M_NCONST + M_NJAC + 1], sv[2 * M_NA];
+    const int tid = threadIdx.x;
+    for (int i = tid; i < M_NPAR; i += CT_PRO_BLOCK) {
+        const double x = P ? P->p[i] : A.params[i];
+        sp[i] = x;
+        if (P) A.params[i] = x;
+    }
+    if (tid == 0 && A.err_reset) *A.err_reset = 0;
     __syncthreads();
+    if ((tid & 31) == 0) {
+        for (int q = tid >> 5; q < M_NPRO; q += CT_PRO_BLOCK / 32) model_prologue(q, sp + 2 * A.nc, sc);
+    } else {
+        for (int a = tid - 1 - (tid >> 5); a < M_NA; a += CT_PRO_BLOCK - CT_PRO_BLOCK / 32) {
+            const int c = A.chain[a];
+            const double r = A.ratio[a];
+            A.vout[2 * a] = sv[2 * a] = sp[c] * r;
+            A.vout[2 * a + 1] = sv[2 * a + 1] = sp[A.nc + c] * r;
+        }
+    }
+    __syncthreads();
+    for (int i = tid; i < M_NCONST + M_NJAC; i += CT_PRO_BLOCK) A.consts[i] = sc[i];
     if (!A.kblock) return;
     CtConsts* K = (CtConsts*)A.kblock;
-    for (int i = threadIdx.x; i < M_NCONST; i += blockDim.x) {
-        const double c = A.consts[i];
+    for (int i = tid; i < M_NCONST; i += CT_PRO_BLOCK) {
+        const double c = sc[i];
         const float h = (float)c;
         K->c[i] = c;
         K->ch[i] = h;
         K->cl[i] = (float)(c - (double)h);
     }
-    for (int i = threadIdx.x; i < 2 * M_NA; i += blockDim.x) {
-        const double v = A.v[i];
-        const float h = (float)v;
-        K->v[i] = v;
-        K->vh[i] = h;
+    for (int i = tid; i < 2 * M_NA; i += CT_PRO_BLOCK) {
+        K->v[i] = sv[i];
+        K->vh[i] = (float)sv[i];
     }
+}
+extern "C" __global__ void __launch_bounds__(CT_PRO_BLOCK) ct_prologue(const __grid_constant__ CtArgs A)
+{
+    ct_prologue_body(A, nullptr);
+}
+extern "C" __global__ void __launch_bounds__(CT_PRO_BLOCK)
+    ct_prologue_host(const __grid_constant__ CtArgs A, const __grid_constant__ CtHostParams P)
+{
+    ct_prologue_body(A, &P);
+}
+// one block per job of a multi-job evaluation
+extern "C" __global__ void __launch_bounds__(CT_PRO_BLOCK) ct_prologue_multi(const CtArgs* __restrict__ jobs)
+{
+    ct_prologue_body(jobs[blockIdx.x], nullptr);
 }
 
 __device__ __forceinline__ void ct_stage_consts(const CtArgs& A, double* sC)

@@ -92,10 +92,12 @@ struct CtHessArgs {
     double* rows;       // [CTAs][CT_HROW]
 };
 
-extern "C" __global__ void ct_hess_prologue(CtHessArgs A)
+// parameter-only constants (one warp per part, up to 16) and couplings
+extern "C" __global__ void __launch_bounds__(512) ct_hess_prologue(CtHessArgs A)
 {
-    if (threadIdx.x == 0) hs_prologue(A.theta, A.img->c);
-    for (int i = threadIdx.x; i < 2 * M_NA; i += blockDim.x) A.img->v[i] = A.v[i];
+    if ((threadIdx.x & 31) == 0)
+        for (int q = threadIdx.x >> 5; q < M_NHPRO; q += 16) hs_prologue(q, A.theta, A.img->c);
+    for (int i = threadIdx.x; i < 2 * M_NA; i += 512) A.img->v[i] = A.v[i];
 }
 
 __device__ __forceinline__ void ct_dmma(double (&c)[2], double a, double b)

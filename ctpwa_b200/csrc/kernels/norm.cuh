@@ -235,17 +235,25 @@ extern "C" __global__ void __launch_bounds__(CT_NORM_BLOCK) ct_norm_build(CtNorm
     }
 }
 
-// Fixed-order column sums of the per-CTA partials: out[2 ne].
+// Fixed-order column sums of the per-CTA partials: out[2 ne]. 32 columns per
+// CTA, its 8 warps on every eighth row (one CTA for all 308 columns of
+// K+K-pi0 and 296 rows, a warp striding down a column at a time: 123 us).
 extern "C" __global__ void __launch_bounds__(256) ct_norm_reduce(const double* __restrict__ partials, int rows, int ne,
                                                                  double* __restrict__ out)
 {
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
-    for (int i = warp; i < 2 * ne; i += nwarp) {
-        double s = 0.0;
-        for (int b = lane; b < rows; b += 32) s += partials[(long long)b * 2 * ne + i];
+    __shared__ double part[8][32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, col = blockIdx.x * 32 + lane;
+    double s = 0.0;
+    if (col < 2 * ne) {
+#pragma unroll 4
+        for (int b = warp; b < rows; b += 8) s += partials[(long long)b * 2 * ne + col];
+    }
+    part[warp][lane] = s;
+    __syncthreads();
+    if (warp == 0 && col < 2 * ne) {
 #pragma unroll
-        for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
-        if (lane == 0) out[i] = s;
+        for (int w = 1; w < 8; ++w) s += part[w][lane];
+        out[col] = s;
     }
 }
 
