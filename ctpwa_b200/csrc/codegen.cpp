@@ -90,30 +90,46 @@ struct Shapes {
         int dn = g.cnst(d);
         return g.mul(poly(L, g.mul(q0v, dn)), g.recip(poly(L, g.mul(q, dn))));
     }
-    // 1 / (m0^2 - m^2 - i m0 G(m)), G = G0 (q/q0)^(2L+1) (m0/m) Bf^2
-    Cx bwr(int m, int m0, int g0, int L, int q, int q0v, double d)
+    // 1 / (m0^2 - m^2 - i m0 G(m)), G = G0 (q/q0)^(2L+1) (m0/m) Bf^2, as
+    // (x + i y) times the real factor `scale` = 1 / (x^2 + y^2). The caller
+    // joins the other real factors to the scale before it multiplies x and y
+    // by it, and y stays one factor: so a chain reads m^2, the event part of
+    // y and that of the real factors, three per-event values (four with the
+    // products y^2 and y times the real factors regrouped by dependence).
+    Cx bwr(int m, int m0, int g0, int L, int q, int q0v, double d, int& scale)
     {
         int x = g.sub(sq(m0), sq(m));
         int thp = g.mul(g.mul(g0, sq(m0)), g.powi(g.recip(q0v), 2 * L + 1));
         int evp = g.mul(g.powi(q, 2 * L + 1), g.recip(m));
-        int y;
         if (L > 0 && L <= 6 && d != 0.0) {
             int dn = g.cnst(d);
             thp = g.mul(thp, poly(L, g.mul(q0v, dn)));
             evp = g.mul(evp, g.recip(poly(L, g.mul(q, dn))));
         }
-        y = g.mul(thp, evp);
-        int is = g.recip(g.add(sq(x), sq(y)));
-        return {g.mul(x, is), g.mul(y, is)};
+        int y = g.keep(g.mul(thp, evp));
+        scale = g.recip(g.add(sq(x), g.square(y)));
+        return {x, y};
+    }
+    Cx bwr(int m, int m0, int g0, int L, int q, int q0v, double d)
+    {
+        int s;
+        Cx c = bwr(m, m0, g0, L, q, q0v, d, s);
+        return {g.mul(c.re, s), g.mul(c.im, s)};
+    }
+    Cx bw(int m, int m0, int g0, int& scale)
+    {
+        int x = g.sub(sq(m0), sq(m)), y = g.mul(m0, g0);
+        scale = g.recip(g.add(sq(x), sq(y)));
+        return {x, y};
     }
     Cx bw(int m, int m0, int g0)
     {
-        int x = g.sub(sq(m0), sq(m)), y = g.mul(m0, g0);
-        int is = g.recip(g.add(sq(x), sq(y)));
-        return {g.mul(x, is), g.mul(y, is)};
+        int s;
+        Cx c = bw(m, m0, g0, s);
+        return {g.mul(c.re, s), g.mul(c.im, s)};
     }
     // Flatte (FlatteC), per-call form: (A - iB) / (A^2 + B^2)
-    Cx flatte(int m, int m0, const std::vector<int>& gs, const std::vector<int>& ch)
+    Cx flatte(int m, int m0, const std::vector<int>& gs, const std::vector<int>& ch, int& scale)
     {
         int s = sq(m);
         // m0^2 - s first: the cancelling pair stays one subtraction
@@ -123,8 +139,8 @@ struct Shapes {
             A = g.add(A, g.mul(gw, g.rho(true, s, ch[2 * i], ch[2 * i + 1])));
             B = g.sub(B, g.mul(gw, g.rho(false, s, ch[2 * i], ch[2 * i + 1])));
         }
-        int iD = g.recip(g.add(sq(A), sq(B)));
-        return {g.mul(A, iD), g.neg(g.mul(B, iD))};
+        scale = g.recip(g.add(sq(A), sq(B)));
+        return {A, g.neg(B)};
     }
     // Flatte, fixed-parameter form (same value, reference arrangement)
     Cx flatteFixed(int m, int m0, const std::vector<int>& gs, const std::vector<int>& ch)
@@ -297,9 +313,11 @@ struct Gen {
         return par;
     }
 
-    // gi: the group (base or permutation variant) whose kinematics are read
-    Cx nodeFactor(const Block& b, int gi, int ni, int s, const std::vector<std::vector<int>>& par)
+    // gi: the group (base or permutation variant) whose kinematics are read;
+    // scale: a real factor of the node kept apart from the complex value returned
+    Cx nodeFactor(const Block& b, int gi, int ni, int s, const std::vector<std::vector<int>>& par, int& scale)
     {
+        scale = G.one();
         const Group& g = m.groups[gi];
         const ModelNode& n = g.nodes[ni];
         int L = n.sls[g.sl_combs[s][ni]].L;
@@ -322,7 +340,8 @@ struct Gen {
             if (match < 0) {
                 if (!n.has_bf) return G.c(1.0);
                 int q0 = S.breakup(G.cnst(n.mass[0] > 0 ? n.mass[0] : 1.0), md1, md2);
-                return G.cr(S.bf(L, qq, q0, n.bf_d));
+                scale = S.bf(L, qq, q0, n.bf_d);
+                return G.c(1.0);
             }
             const ResInstance& R = b.res[match];
             const auto& P = par[match];
@@ -334,11 +353,20 @@ struct Gen {
                 return k == 0 ? md1 : md2;
             };
             int q0r = S.q0(m0, dep(0), dep(1));
-            Cx bfx = R.has_bf ? G.cr(S.bf(L, qq, q0r, R.d)) : G.c(1.0);
+            const int bfr = R.has_bf ? S.bf(L, qq, q0r, R.d) : G.one();
+            Cx bfx = G.cr(bfr);
             switch (R.type) {
-            case ModelType::BWR: return G.cmul(S.bwr(mm, P[0], P[1], R.Lmin, qq, q0r, R.has_bf ? R.d : 0.0), bfx);
-            case ModelType::BW: return S.bw(mm, P[0], P[1]);
-            case ModelType::ONE: return bfx;
+            case ModelType::BWR: {
+                int is;
+                Cx c = S.bwr(mm, P[0], P[1], R.Lmin, qq, q0r, R.has_bf ? R.d : 0.0, is);
+                scale = G.mul(is, bfr);
+                return c;
+            }
+            case ModelType::BW:
+                return S.bw(mm, P[0], P[1], scale);
+            case ModelType::ONE:
+                scale = bfr;
+                return G.c(1.0);
             case ModelType::Flatte: {
                 std::vector<int> gs, ch;
                 for (size_t i = 0; i < R.channels.size(); ++i) {
@@ -346,7 +374,10 @@ struct Gen {
                     ch.push_back(G.cnst(R.channels[i].first));
                     ch.push_back(G.cnst(R.channels[i].second));
                 }
-                return G.cmul(S.flatte(mm, P[0], gs, ch), bfx);
+                int is;
+                Cx c = S.flatte(mm, P[0], gs, ch, is);
+                scale = G.mul(is, bfr);
+                return c;
             }
             case ModelType::GS: {
                 double mpi = R.channels.empty() ? 0.1396 : R.channels[0].first;
@@ -1518,7 +1549,13 @@ GeneratedModel generateModel(const Model& m)
         for (int s = 0; s < gr.nSL(); ++s)
             for (int v : vars) {
                 Cx F = g.G.c(m.groups[v].sign);
-                for (size_t ni = 0; ni < gr.nodes.size(); ++ni) F = g.G.cmul(F, g.nodeFactor(b, v, (int)ni, s, par));
+                int scale = g.G.one();
+                for (size_t ni = 0; ni < gr.nodes.size(); ++ni) {
+                    int sc;
+                    F = g.G.cmul(F, g.nodeFactor(b, v, (int)ni, s, par, sc));
+                    scale = g.G.mul(scale, sc);
+                }
+                F = g.G.cscale(F, g.G.keepLog(scale));
                 Gen::TermOut t;
                 t.col = b.site + s;
                 t.plane = g.out.group_plane0[v] + s;

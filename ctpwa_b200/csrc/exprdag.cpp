@@ -128,7 +128,7 @@ int Graph::mul(int a, int b)
         while (!st.empty()) {
             auto [x, depth] = st.back();
             st.pop_back();
-            if (nodes[x].op == Mul && cls(x) == (DEP_THETA | DEP_EVENT) && depth < 3) {
+            if (nodes[x].op == Mul && cls(x) == (DEP_THETA | DEP_EVENT) && depth < 3 && !kept_.count(x)) {
                 st.push_back({nodes[x].a, depth + 1});
                 st.push_back({nodes[x].b, depth + 1});
             } else {
@@ -254,6 +254,15 @@ int Graph::powi(int a, int n)
     return (n % 2) ? mul(h2, a) : h2;
 }
 
+int Graph::dlog(int a, int j)
+{
+    const Node nd = nodes[a];
+    if (!(nd.dep & DEP_THETA)) return zero_;
+    if (nd.op == Mul && nd.dep != DEP_THETA) return add(dlog(nd.a, j), dlog(nd.b, j));
+    if (nd.op == Recip) return neg(mul(a, deriv(nd.a, j)));
+    return mul(deriv(a, j), recip(a));
+}
+
 int Graph::deriv(int n, int j)
 {
     const Node nd = nodes[n];
@@ -262,6 +271,11 @@ int Graph::deriv(int n, int j)
     auto it = dmemo_.find(key);
     if (it != dmemo_.end()) return it->second;
     int r = zero_;
+    // n times a logarithmic derivative, n staying one factor
+    auto scaled = [&](int l) {
+        if (!isConst(l)) return mulRaw(n, l);
+        return val(l) == 0.0 ? zero_ : mul(n, l);
+    };
     switch (nd.op) {
     case Const:
     case Kin:
@@ -270,7 +284,16 @@ int Graph::deriv(int n, int j)
     case Theta: r = nd.idx == j ? one_ : zero_; break;
     case Add: r = add(deriv(nd.a, j), deriv(nd.b, j)); break;
     case Sub: r = sub(deriv(nd.a, j), deriv(nd.b, j)); break;
-    case Mul: r = add(mul(deriv(nd.a, j), nd.b), mul(nd.a, deriv(nd.b, j))); break;
+    case Mul:
+        if (log_.count(n)) {
+            r = scaled(dlog(n, j));
+        } else if (log_.count(nd.a) || log_.count(nd.b)) {
+            const int s = log_.count(nd.a) ? nd.a : nd.b, x = s == nd.a ? nd.b : nd.a;
+            r = add(mul(deriv(x, j), s), scaled(dlog(s, j)));
+        } else {
+            r = add(mul(deriv(nd.a, j), nd.b), mul(nd.a, deriv(nd.b, j)));
+        }
+        break;
     case Recip: r = neg(mul(mul(n, n), deriv(nd.a, j))); break;
     case Neg: r = neg(deriv(nd.a, j)); break;
     case Sqrt: r = mul(mul(cnst(0.5), deriv(nd.a, j)), recip(n)); break;
@@ -286,6 +309,8 @@ int Graph::deriv(int n, int j)
     }
     case Sel: r = sel((Cmp)nd.cmp, nd.c, deriv(nd.a, j), deriv(nd.b, j)); break;
     }
+    // the derivative of a kept product is one factor too
+    if (kept_.count(n) && !log_.count(n) && nodes[r].op == Mul) keep(r);
     dmemo_[key] = r;
     return r;
 }

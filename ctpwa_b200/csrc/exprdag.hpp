@@ -15,6 +15,7 @@
 #include <cstdint>
 #include <map>
 #include <memory>
+#include <set>
 #include <string>
 #include <tuple>
 #include <unordered_map>
@@ -96,6 +97,22 @@ public:
     int sel(Cmp cmp, int c, int a, int b);
     int rho(bool im, int s, int ma, int mb);
     int powi(int a, int n);
+    // a product that stays one factor: mul() does not regroup its parts into
+    // the products it joins, nor those of its square
+    int keep(int a)
+    {
+        kept_.insert(a);
+        return a;
+    }
+    // a kept product of non-zero factors whose derivative is formed from its
+    // logarithm: d(x S) = dx S + (x S) dlog S shares x S with the value, and
+    // dlog(1 / s) = -(1 / s) ds, dlog of a parameter-only factor one constant
+    int keepLog(int a)
+    {
+        log_.insert(a);
+        return keep(a);
+    }
+    int square(int a) { return kept_.count(a) ? mulRaw(a, a) : mul(a, a); }
     int recip(int a);
     int zero() { return zero_; }
     int one() { return one_; }
@@ -141,6 +158,8 @@ private:
     int make(Node n);
     int mulRaw(int a, int b);  // a * b as one node, no regrouping
     int zero_, one_;
+    std::set<int> kept_, log_;
+    int dlog(int a, int j);  // d log(a) / d theta_j of a product
     std::map<std::tuple<int, int, int, int, int, double, int>, int> memo_;
     std::map<std::pair<int, int>, int> dmemo_;
 };
