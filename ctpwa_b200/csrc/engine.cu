@@ -548,7 +548,7 @@ __device__ __forceinline__ void ct_sum_rows(const FinalizeArgs& A, const double*
     __syncthreads();
 }
 // rows of doubles of wsum: all three samples at once (their loads in flight
-// together: the finalize of 296 rows 8.5 -> TODO us) while they fit, else one by one
+// together: three passes with two barriers each before) while they fit, else one by one
 __host__ __device__ __forceinline__ int ct_sum_samples(int nacc) { return nacc <= 200 ? 3 : 1; }
 
 // Per-sample sums of the partial rows plus the sample totals (event-sharded
@@ -990,8 +990,8 @@ Engine::Engine(const std::string& config_path, const EngineOptions& opt) : opt_(
         bool all = !k_ang_.empty();
         for (void* k : k_ang_) all = all && k;
         if (all && npair > 0 && nplane * npair <= 32) {
-            alloc(d_pairmax_, sizeof(unsigned long long) * (2 * nplane * npair + 1));
-            CT_CUDA(cudaMemsetAsync(d_pairmax_, 0, sizeof(unsigned long long) * (2 * nplane * npair + 1), init_stream_));
+            alloc(d_pairmax_, sizeof(unsigned long long) * (2 * nplane * npair + 3));
+            CT_CUDA(cudaMemsetAsync(d_pairmax_, 0, sizeof(unsigned long long) * (2 * nplane * npair + 3), init_stream_));
         }
     }
     for (int k = 0; k < 3; ++k)
@@ -1310,14 +1310,15 @@ std::string angularSource(const std::vector<AgGroupHost>& gh, const std::vector<
         const int npair = A.npol / 2;
         // pairmax (may be null): maxima over events of
         // |SL_{c,npol-1-q} -+ conj(SL_{c,q})| at [(c npair + q) 2 + 0 / 1] and
-        // of |SL| at [2 nplane npair] (the layout of ct_pair_check_kernel),
+        // of |SL| at [2 nplane npair], then of |Re SL| and |Im SL| of the
+        // polarisation paired with itself (the layout of ct_pair_check_kernel),
         // accumulated by one atomic per warp and value
         o << "extern \"C\" __global__ void __launch_bounds__(128) ct_ang_" << gi
           << "(const double* __restrict__ p4, long long n, long long ld, AgTables T, double2* __restrict__ out64,\n"
              "    float2* __restrict__ out32, double* __restrict__ kin, unsigned long long* __restrict__ pairmax)\n{\n"
              "  const long long e = (long long)blockIdx.x * 128 + threadIdx.x;\n";
         if (npair > 0) {
-            o << "  double pm[" << std::max(1, 2 * A.nsl * npair) << "] = {}, big = 0.0;\n";
+            o << "  double pm[" << std::max(1, 2 * A.nsl * npair) << "] = {}, big = 0.0, mid[2] = {};\n";
             o << "  if (e < n) {\n";
         } else {
             o << "  if (e >= n) return;\n  {\n";
@@ -1414,6 +1415,11 @@ std::string angularSource(const std::vector<AgGroupHost>& gh, const std::vector<
                 for (int p = 0; p < A.npol; ++p)
                     o << "    big = fmax(big, agDist(c" << last << "[" << srcs[p] << "].x, c" << last << "[" << srcs[p]
                       << "].y));\n";
+                if (A.npol % 2) {
+                    const std::string c = "c" + std::to_string(last) + "[" + std::to_string(srcs[npair]) + "]";
+                    o << "    mid[0] = fmax(mid[0], agDist(" << c << ".x, 0.0)); mid[1] = fmax(mid[1], agDist(" << c
+                      << ".y, 0.0));\n";
+                }
                 for (int q = 0; q < npair; ++q) {
                     const std::string a = "c" + std::to_string(last) + "[" + std::to_string(srcs[q]) + "]",
                                       b = "c" + std::to_string(last) + "[" + std::to_string(srcs[A.npol - 1 - q]) + "]";
@@ -1437,8 +1443,11 @@ std::string angularSource(const std::vector<AgGroupHost>& gh, const std::vector<
                         o << "    { const double v = agWarpMax(pm[" << k << "]); if (lane == 0) atomicMax(pairmax + " << out
                           << ", (unsigned long long)__double_as_longlong(v)); }\n";
                     }
-            o << "    { const double v = agWarpMax(big); if (lane == 0) atomicMax(pairmax + " << 2 * nplane * npair
-              << ", (unsigned long long)__double_as_longlong(v)); }\n  }\n";
+            for (int w = 0; w < 3; ++w)
+                o << "    { const double v = agWarpMax(" << (w == 0 ? "big" : w == 1 ? "mid[0]" : "mid[1]")
+                  << "); if (lane == 0) atomicMax(pairmax + " << 2 * nplane * npair + w
+                  << ", (unsigned long long)__double_as_longlong(v)); }\n";
+            o << "  }\n";
         }
         o << "}\n\n";
     }
@@ -1612,47 +1621,61 @@ __global__ void ct_pair_check_kernel(const double2* __restrict__ sl, long long n
                 atomicMax(out + (c * npair + q) * 2 + 1, (unsigned long long)__double_as_longlong(dn));
             }
         }
-    double big = 0.0;
+    double m[3] = {0.0, 0.0, 0.0};
     for (int r = 0; r < nplane * npol; ++r) {
         const double2* __restrict__ ra = sl + (long long)r * ld;
-        for (long long e = e0; e < n; e += stride) big = fmax(big, ct_dist(ra[e].x, ra[e].y));
+        const bool self = npol % 2 && r % npol == npair;
+        for (long long e = e0; e < n; e += stride) {
+            m[0] = fmax(m[0], ct_dist(ra[e].x, ra[e].y));
+            if (self) {
+                m[1] = fmax(m[1], ct_dist(ra[e].x, 0.0));
+                m[2] = fmax(m[2], ct_dist(ra[e].y, 0.0));
+            }
+        }
     }
-    big = ct_warp_max(big);
-    if (lane == 0) atomicMax(out + 2 * nplane * npair, (unsigned long long)__double_as_longlong(big));
+    for (int w = 0; w < 3; ++w) {
+        const double v = ct_warp_max(m[w]);
+        if (lane == 0) atomicMax(out + 2 * nplane * npair + w, (unsigned long long)__double_as_longlong(v));
+    }
 }
 
 }  // namespace
+
+// The FP64 table of paired polarisations from the full one ([plane][pol][ld]
+// complex): per plane x and y of polarisations p < npol / 2, then the one
+// paired with itself (its real part, or mid_im its imaginary part), each a row
+// [ld].
+__global__ void __launch_bounds__(256) ct_paired_rows_kernel(const double2* __restrict__ full, long long n, long long ld,
+                                                             int nplane, int npol, int mid_im,
+                                                             double* __restrict__ out)
+{
+    const int ns = (npol + 1) / 2;
+    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < n; e += (long long)gridDim.x * blockDim.x)
+        for (int c = 0; c < nplane; ++c)
+            for (int p = 0; p < ns; ++p) {
+                const double2 x = full[(long long)(c * npol + p) * ld + e];
+                out[(long long)(c * npol + 2 * p) * ld + e] = 2 * p + 1 == npol && mid_im ? x.y : x.x;
+                if (2 * p + 1 < npol) out[(long long)(c * npol + 2 * p + 1) * ld + e] = x.y;
+            }
+}
 
 // Decides whether the polarisations pair up as SL_{npol-1-q} = conj(SL_q) on
 // every event of the phase-space, data and background samples (to 1e-12 of
 // the largest |SL|; e.g. the M = -1 and M = +1 states of a J/psi decaying to
 // spin-0 particles), and if so switches the fused kernels to their paired
-// variants (ct_fused_*_pc) with compact tables holding polarisations
-// 0 .. (npol+1)/2 - 1: the FP32 table is replaced, the plain kernel gets an
-// FP64 copy (the other kernels keep the full FP64 table). The check also
-// measures the minus-sign relation, which the paired kernels do not use.
-// Runs on the constructor's initialisation stream.
-// the compact table of paired polarisations, event-major:
-// out[e][c ns + q] = rows[c npol + q][e] (q < ns stored polarisations; zeros
-// for the padding events past n)
-__global__ void ct_compact_event_major_kernel(const double2* __restrict__ rows, long long n, long long ld, int nplane,
-                                              int npol, int ns, double2* __restrict__ out)
-{
-    const int nr = nplane * ns;
-    for (long long e = blockIdx.x * (long long)blockDim.x + threadIdx.x; e < ld; e += (long long)gridDim.x * blockDim.x)
-        for (int c = 0; c < nplane; ++c)
-            for (int q = 0; q < ns; ++q)
-                out[e * nr + c * ns + q] = e < n ? rows[(long long)(c * npol + q) * ld + e] : make_double2(0.0, 0.0);
-}
-
+// variants (ct_fused_*_pc) with compact tables: the FP32 table is replaced by
+// polarisations 0 .. (npol+1)/2 - 1, the plain and Hessian kernels get an
+// FP64 table of reals (ct_paired_rows_kernel; the other kernels keep the full
+// FP64 table). The check also measures the minus-sign relation, which the
+// paired kernels do not use. Runs on the constructor's initialisation stream.
 void Engine::pairPolarisations()
 {
     const int npol = model_.npol, nplane = gen_.nplane, npair = npol / 2;
     const char* off = std::getenv("CTPWA_NO_POL_PAIRING");
     if (!opt_.pair_polarisations || npair == 0 || nplane * npair > 32 || (off && *off && *off != '0')) return;
-    const int nout = 2 * nplane * npair + 1;
+    const int nout = 2 * nplane * npair + 3;
     std::vector<double> worst(2 * nplane * npair, 0.0);
-    double big = 0.0;
+    double big = 0.0, mid[2] = {0.0, 0.0};
     if (d_pairmax_) {
         // gathered by the generated angular kernels over all three samples
         std::vector<unsigned long long> h(nout);
@@ -1661,6 +1684,7 @@ void Engine::pairPolarisations()
         CT_CUDA(cudaStreamSynchronize(init_stream_));
         for (int i = 0; i < 2 * nplane * npair; ++i) std::memcpy(&worst[i], &h[i], sizeof(double));
         std::memcpy(&big, &h[2 * nplane * npair], sizeof(double));
+        std::memcpy(mid, &h[2 * nplane * npair + 1], 2 * sizeof(double));
     }
     unsigned long long* d_out = nullptr;
     if (!d_pairmax_) alloc(d_out, sizeof(unsigned long long) * nout);
@@ -1679,9 +1703,10 @@ void Engine::pairPolarisations()
             std::memcpy(&x, &h[i], sizeof(double));
             worst[i] = std::max(worst[i], x);
         }
-        double b;
-        std::memcpy(&b, &h[2 * nplane * npair], sizeof(double));
-        big = std::max(big, b);
+        double b[3];
+        std::memcpy(b, &h[2 * nplane * npair], 3 * sizeof(double));
+        big = std::max(big, b[0]);
+        for (int w = 0; w < 2; ++w) mid[w] = std::max(mid[w], b[1 + w]);
     }
     devFree(d_out);
     const double tol = 1e-12 * big;
@@ -1697,21 +1722,29 @@ void Engine::pairPolarisations()
     // the paired kernels rebuild conjugates with a plus sign
     if (!ok || neg != 0) return;
     const int ns = (npol + 1) / 2;
-    paired_[0] = true;
+    // The FP64 kernels read the polarisation paired with itself as a real
+    // number: parity makes it real or imaginary, in all planes alike, and a
+    // phase common to a polarisation changes neither |S_p|^2 nor any gradient.
+    const bool mid_im = npol % 2 && mid[1] > tol;
+    paired_[0] = npol % 2 == 0 || mid[0] <= tol || mid[1] <= tol;
     paired_[1] = opt_.mixed_tables;
     for (int pr = 0; pr < 2; ++pr)
         if (paired_[pr]) (pr == 0 ? k_f64_ : k_mixed_) = k_pc_[pr];
+    if (paired_[0]) {
+        shape_.stage[0] = shape_.stage_pc;
+        shape_.dsmem[0] = shape_.dsmem_pc;
+    }
     for (int k = 0; k < 3; ++k) {
         DeviceSample& d = samples_[k];
         if (!d.slamp64) continue;
         const size_t rows = (size_t)nplane * ns;
         if (paired_[0]) {
-            // the compact FP64 table event-major: [ld][plane x stored polarisation]
-            alloc(d.slamp64p, sizeof(double2) * rows * d.ld);
-            device_bytes_ += sizeof(double2) * rows * d.ld;
+            const size_t bytes = sizeof(double) * (size_t)nplane * npol * d.ld;
+            alloc(d.slamp64p, bytes);
+            device_bytes_ += bytes;
             const unsigned grid = (unsigned)std::min<long long>((d.ld + 255) / 256, 148LL * 16);
-            ct_compact_event_major_kernel<<<grid, 256, 0, init_stream_>>>(d.slamp64, d.n, d.ld, nplane, npol, ns,
-                                                                           d.slamp64p);
+            ct_paired_rows_kernel<<<grid, 256, 0, init_stream_>>>(d.slamp64, d.n, d.ld, nplane, npol, mid_im,
+                                                                   d.slamp64p);
             CT_CUDA(cudaGetLastError());
         }
         if (paired_[1] && d.slamp32) {
@@ -1887,18 +1920,18 @@ FusedShape fusedShape(const GeneratedModel& gen)
 
     for (int i = 0; i < 2; ++i)
         if (sh.block[i] % 32) throw std::runtime_error("fused block sizes must be multiples of 32");
-    // Staging of the event tables through shared memory, used when its two
+    // Staging of the event tables through shared memory, used when its
     // buffers fit at the requested residency next to the static shared
     // memory: 1 the frontier rows and 2 the frontier and angular rows, by
     // per-warp bulk copies of 32-event tiles; 3 the frontier values by
-    // per-thread asynchronous copies of the next event's values. CTPWA_STAGE
-    // sets it for both kernels. Default: 3 for the mixed form (K+K-pi0:
-    // 0.52-0.53 ms, against 0.63 ms direct, 0.744 ms with mode 1 and 1.10 ms
-    // with mode 2 at 1 CTA per SM), off for the plain path (its gradient-sum
-    // slots leave no room for the buffers at 2 CTAs per SM; with the slots
-    // in registers instead, mode 3 measured 1.39 ms against 1.15 ms).
-    const int st = get("CTPWA_STAGE", -1, 0, 3);
-    const int stage_req[2] = {st >= 0 ? st : 0, st >= 0 ? st : 3};
+    // per-thread asynchronous copies of the next event's values; 4 (plain
+    // path) the frontier and angular values likewise, one buffer each.
+    // CTPWA_STAGE sets it for both kernels. Default: 3 for the mixed form
+    // (K+K-pi0: 0.52-0.53 ms, against 0.63 ms direct, 0.744 ms with mode 1
+    // and 1.10 ms with mode 2 at 1 CTA per SM), 4 for the plain path
+    // (0.561 ms against 0.709 ms direct), direct loads where the buffers do not fit.
+    const int st = get("CTPWA_STAGE", -1, 0, 4);
+    const int stage_req[2] = {st >= 0 ? st : 4, st >= 0 && st < 4 ? st : 3};
     const long long rowb[2] = {16, 8};  // bytes per complex angular value (FP64, FP32)
     const long long accb[2] = {8, 4};   // bytes per gradient sum (FP64, FP32)
     const long long per_sm = 228LL * 1024, per_cta = 227LL * 1024, reserve = 8LL * 1024;
@@ -1922,8 +1955,14 @@ FusedShape fusedShape(const GeneratedModel& gen)
             const long long na = i == 0 ? gen.nev64 : evfStride(gen), nb = i == 0 ? 0 : gen.nevd, sz = i == 0 ? 8 : 4;
             stage_bytes = (2LL * std::max(1LL, na) * sh.block[i] * sz + 15) / 16 * 16 + 2LL * nb * sh.block[i] * 8;
         }
+        if (stage_on == 4) stage_bytes = (npl * rowb[0] + 8LL * gen.nev64) * sh.block[0];
         if (stage_on && fits(i, acc_bytes + stage_bytes)) sh.stage[i] = stage_on;
         sh.dsmem[i] = (int)(acc_bytes + (sh.stage[i] ? stage_bytes : 0));
+        if (i == 0) {
+            if (stage_on == 4) stage_bytes = (npl + gen.nev64) * 8LL * sh.block[0];
+            if (stage_on && fits(0, acc_bytes + stage_bytes)) sh.stage_pc = stage_on;
+            sh.dsmem_pc = (int)(acc_bytes + (sh.stage_pc ? stage_bytes : 0));
+        }
     }
     return sh;
 }
@@ -2026,6 +2065,7 @@ std::string jitCubin(const GeneratedModel& gen, bool* cache_hit)
     optv.push_back("-DCT_F64_ACC=" + std::to_string(sh.acc[0]));
     optv.push_back("-DCT_MX_ACC=" + std::to_string(sh.acc[1]));
     optv.push_back("-DCT_F64_STAGE=" + std::to_string(sh.stage[0]));
+    optv.push_back("-DCT_F64_PC_STAGE=" + std::to_string(sh.stage_pc));
     optv.push_back("-DCT_MX_STAGE=" + std::to_string(sh.stage[1]));
 
     optv.push_back("-DCT_F64_BLOCK=" + std::to_string(sh.block[0]));
@@ -2057,6 +2097,7 @@ std::string jitHvpCubin(const GeneratedModel& gen, bool paired, bool* cache_hit)
     optv.push_back(std::string("-DCT_HVP_PAIRED=") + (paired ? "1" : "0"));
     return nvrtcCubin("#include \"hessian.cuh\"\n",
                       {{"device_helpers.cuh", readFile(dir + "/device_helpers.cuh")},
+                       {"angular_load.cuh", readFile(dir + "/angular_load.cuh")},
                        {"hessian.cuh", readFile(dir + "/hessian.cuh")},
                        {"model.cuh", gen.header},
                        {"model_dual.cuh", gen.dual_header}},
@@ -2096,6 +2137,7 @@ std::string jitHessCubin(const GeneratedModel& gen, bool paired, bool* cache_hit
     optv.push_back(std::string("-DCT_HESS_PAIRED=") + (paired ? "1" : "0"));
     return nvrtcCubin("#include \"hessgram.cuh\"\n",
                       {{"device_helpers.cuh", readFile(dir + "/device_helpers.cuh")},
+                       {"angular_load.cuh", readFile(dir + "/angular_load.cuh")},
                        {"hessgram.cuh", readFile(dir + "/hessgram.cuh")},
                        {"model.cuh", gen.header},
                        {"model_hess.cuh", gen.hess_header}},
@@ -2149,7 +2191,7 @@ std::string shapeKey(const FusedShape& sh)
 {
     std::string k;
     for (int i = 0; i < 2; ++i)
-        for (int v : {sh.block[i], sh.minb[i], sh.acc[i], sh.stage[i]}) k += std::to_string(v) + " ";
+        for (int v : {sh.block[i], sh.minb[i], sh.acc[i], sh.stage[i], sh.stage_pc}) k += std::to_string(v) + " ";
     return k;
 }
 
@@ -2212,9 +2254,10 @@ void Engine::compileKernel()
     CT_CUDA(cudaLibraryGetKernel(&kprom, lib, "ct_prologue_multi"));
     k_pro_multi_ = (void*)kprom;
     for (int pr = 0; pr < 2; ++pr)
-        if (shape_.dsmem[pr] > 0)
+        if (shape_.dsmem[pr] > 0 || (pr == 0 && shape_.dsmem_pc > 0))
             for (void* k : {pr == 0 ? k_f64_ : k_mixed_, k_pc_[pr], k_multi_[pr][0], k_multi_[pr][1]})
-                CT_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize, shape_.dsmem[pr]));
+                CT_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             std::max(shape_.dsmem[pr], pr == 0 ? shape_.dsmem_pc : 0)));
     k_int_ = (void*)kin;
     {
         std::string key = gen_.id;
@@ -2824,7 +2867,7 @@ void Engine::hessian(const double* d_params, double* d_hess, double rel_step, cu
 
 // argument block of the Hessian-vector-product kernels (must match CtHvpArgs)
 struct CtHvpSampleH {
-    const double2* slamp;
+    const void* slamp;
     const double* ev;
     const double* w;
     long long n;
@@ -2853,7 +2896,7 @@ struct CtHvpArgsH {
 
 // argument blocks of the one-pass Hessian kernels (must match kernels/hessgram.cuh)
 struct CtHessSampleH {
-    const double2* slamp;
+    const void* slamp;
     const double* ev;
     const double* w;
     long long n;
@@ -3128,7 +3171,7 @@ void Engine::hessSums(const double* d_params, const double* d_dirs, int ndir, do
         if (hess_lay_[k][1] == 0) continue;
         CtHessSampleH& sm = a.s[a.nsamp++];
         const DeviceSample& d = samples_[k % 3];
-        sm.slamp = paired_[0] ? d.slamp64p : d.slamp64;
+        sm.slamp = paired_[0] ? (const void*)d.slamp64p : (const void*)d.slamp64;
         sm.ev = d.ev64;
         sm.w = k == 0 ? nullptr : d.w;
         sm.n = d.n;
@@ -3201,7 +3244,7 @@ void Engine::forwardHvpSums(const double* d_params, const double* d_dirs, int nd
         if (hlay_.cta[k][1] == 0) continue;
         CtHvpSampleH& sm = a.s[ns++];
         const DeviceSample& d = samples_[k];
-        sm.slamp = paired_[0] ? d.slamp64p : d.slamp64;
+        sm.slamp = paired_[0] ? (const void*)d.slamp64p : (const void*)d.slamp64;
         sm.ev = d.ev64;
         sm.w = d.w;
         sm.n = d.n;

@@ -28,6 +28,11 @@ struct FusedShape {
     int stage[2] = {0, 0};
     int acc[2] = {1, 0};  // per-thread gradient sums in shared memory
     int dsmem[2] = {0, 0};
+    // the plain kernel's variant for paired polarisations, whose angular
+    // records are smaller; they become stage[0] and dsmem[0] once the samples
+    // are found to be paired
+    int stage_pc = 0;
+    int dsmem_pc = 0;
 };
 FusedShape fusedShape(const GeneratedModel& gen);
 
@@ -37,7 +42,7 @@ struct DeviceSample {
     double* p4 = nullptr;      // SoA [n_final * 4][n]
     double2* slamp64 = nullptr;  // [nplane * npol][ld]
     float2* slamp32 = nullptr;   // mixed-precision copy (polarisation-paired when the engine pairs them)
-    double2* slamp64p = nullptr; // polarisation-paired FP64 copy for the plain fused kernel
+    double* slamp64p = nullptr;  // polarisation-paired FP64 copy (rows of reals) for the plain fused and Hessian kernels
     double* kin = nullptr;     // [nkin][ld] kinematic cache (initialisation only)
     double* ev64 = nullptr;    // [nev64][ld] frontier values, FP64
     float* evf = nullptr;      // [nevf][ld] mixed form, FP32 frontier values

@@ -63,11 +63,15 @@ template <typename L>
 constexpr int ct_nsum = 2 * M_NA + (sizeof(L) == 8 ? M_NADJ : M_NTH);
 
 // shared-memory staging of the event tables: 0 off; by per-warp bulk copies
-// 1 the frontier rows, 2 the frontier and angular rows; 3 the frontier values
-// by per-thread asynchronous copies (the host sets it when the two buffers
-// fit at the requested residency)
+// 1 the frontier rows, 2 the frontier and angular rows; by per-thread
+// asynchronous copies 3 the frontier values (two buffers), 4 the frontier and
+// angular values (one buffer each); the host sets it when the buffers fit at
+// the requested residency
 #ifndef CT_F64_STAGE
 #define CT_F64_STAGE 0
+#endif
+#ifndef CT_F64_PC_STAGE  // the variant for paired polarisations
+#define CT_F64_PC_STAGE CT_F64_STAGE
 #endif
 #ifndef CT_MX_STAGE
 #define CT_MX_STAGE 0
@@ -84,7 +88,7 @@ constexpr int ct_nsum = 2 * M_NA + (sizeof(L) == 8 ? M_NADJ : M_NTH);
 #endif
 
 struct CtSample {
-    const void* slamp;  // full FP64: [M_NPLANE * M_NPOL planes][ld] of SL2; FP32 and paired FP64: event-major records
+    const void* slamp;  // FP64: [M_NPLANE * M_NPOL][ld] complex, or real when paired; FP32: event-major records
     const void* ev;     // frontier rows [M_NEV][ld] FP64 (plain), [M_NEVF][ld] FP32 (mixed)
     const double* evd;  // mixed form: FP64 frontier rows [M_NEVD][ld]
     const double* w;    // per-event weights or nullptr (unit weights)
@@ -126,12 +130,18 @@ struct CtArgs {
 // Conjugate-paired polarisations: when every event satisfies
 // SL_{plane, npol-1-q} = conj(SL_{plane, q}) (checked on all samples when they
 // are loaded), the angular tables of the fused kernels store the first
-// CT_NPOL_STORED polarisations only, [plane][q][ld], and the *_pc kernels
-// rebuild the others as conjugates (the negation folds into the FMAs).
+// CT_NPOL_STORED polarisations only, and the *_pc kernels rebuild the others
+// as conjugates (the negation folds into the FMAs). The polarisation paired
+// with itself (npol odd) is real or imaginary, and its phase drops out, so the
+// FP64 table keeps one real for it: M_NPOL reals per plane,
+// [plane][x, y of each pair, the real][ld] (K+K-pi0: 120 instead of 160 bytes
+// per event).
 #define CT_NPOL_STORED ((M_NPOL + 1) / 2)
 // The FP32 angular table is event-major: each event's NPL complex values
 // (NPL = M_NPLANE x the stored polarisations) in one record of an even
-// number of float2, read as float4; the FP64 tables are [row][ld].
+// number of float2, read as float4; the FP64 tables are [row][ld], so that a
+// warp's copy of a value to shared memory is one contiguous segment (16-byte
+// copies from 160-byte records took the shared-memory pipe to 67 %).
 #define CT_SL32_STRIDE(NPL) (((NPL) + 1) / 2 * 2)
 
 // Per-call constants of the fused kernels in the constant bank: the
@@ -151,7 +161,7 @@ __constant__ CtConsts ct_k;
 // One call's inputs from its parameters, by one CTA: the couplings
 // v_a = ratio_a p_chain(a), the parameter-only part of every lineshape with
 // the Jacobian of the adjoint constants (one thread of a warp per part: the
-// dependent FP64 chains run side by side, 5.3 -> 2.6 us on three chains of rho), and
+// dependent FP64 chains run side by side), and
 // the constant-bank image. P: the parameters come with the launch and are
 // stored to A.params for the finalize, without a copy ahead of the kernel.
 #define CT_PRO_BLOCK 512
@@ -225,6 +235,16 @@ struct CtVec2<double> {
 template <>
 struct CtVec2<float> {
     typedef float2 type;
+};
+
+// element of the angular table: complex, but real in the paired FP64 table
+template <typename R, bool PAIRED>
+struct CtSlElem {
+    typedef typename CtVec2<R>::type type;
+};
+template <>
+struct CtSlElem<double, true> {
+    typedef double type;
 };
 
 // CTA reduction of the per-thread accumulators: two FP64 sums (log-likelihood
@@ -434,15 +454,15 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
     const CtSample& S = A.s[si];
     const int kind = PH_ONLY ? 0 : S.kind;
     const long long n = S.n;
-    const SL2* __restrict__ slamp = (const SL2*)S.slamp;
     // this event's angular values: its record of the event-major FP32 table,
-    // or its first value of the [row][ld] FP64 table
-    // (event-major: the FP32 table, and the compact FP64 table of paired
-    // polarisations; the full FP64 table is [row][ld])
-    constexpr int SL_NPL = M_NPLANE * (PAIRED ? CT_NPOL_STORED : M_NPOL);
-    constexpr bool SL_EM = sizeof(R) == 4 || PAIRED;
-    constexpr int SL_SLS = sizeof(R) == 4 ? CT_SL32_STRIDE(SL_NPL) : SL_NPL;
-    auto slat = [&](long long e) -> const SL2* { return SL_EM ? slamp + e * SL_SLS : slamp + e; };
+    // or its first value of the [row][ld] FP64 table (rows of reals when paired)
+    constexpr bool SL_REAL = sizeof(R) == 8 && PAIRED;
+    typedef typename CtSlElem<R, PAIRED>::type SLT;
+    const SLT* __restrict__ slamp = (const SLT*)S.slamp;
+    constexpr int SL_NPL = M_NPLANE * (PAIRED && !SL_REAL ? CT_NPOL_STORED : M_NPOL);
+    constexpr bool SL_EM = sizeof(R) == 4;
+    constexpr int SL_SLS = SL_EM ? CT_SL32_STRIDE(SL_NPL) : SL_NPL;
+    auto slat = [&](long long e) -> const SLT* { return SL_EM ? slamp + e * SL_SLS : slamp + e; };
     const L* __restrict__ eva = (const L*)S.ev;
     const double* __restrict__ evb = S.evd;
     const double* __restrict__ wts = S.w;
@@ -473,17 +493,22 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
     // all per-event work: ap / bp / slp point at this event's frontier values
     // (table type, FP64) and angular values, consecutive values `ks` / `ss`
     // elements apart
-    auto event = [&](long long e, const L* __restrict__ ap, const double* __restrict__ bp, long long ks,
-                     const SL2* __restrict__ slp, long long ss) {
+    // (frontier_read, angular_due and angular_read mark the points where the
+    // event's frontier values are in registers, where its angular values are
+    // first needed, and where they are in registers)
+    auto event = [&](long long e, const L* ap, const double* bp, long long ks, const SLT* slp, long long ss,
+                     auto frontier_read, auto angular_due, auto angular_read) {
         // ---- lineshapes with parameter derivatives ----
         CtEvent<L> ev;
         ev.load(ap, bp, ks);
+        frontier_read();
         auto mid = [&](const L* Fr, const L* Fi, L* Wr, L* Wi) -> bool {
         // ---- coherent sum over amplitudes ----
         // (paired tables: SL_{c,NPOL-1-p} = conj(SL_{c,p}), only the first
         // CT_NPOL_STORED polarisations are stored and read)
         constexpr int NPS = PAIRED ? CT_NPOL_STORED : M_NPOL;
         SL2 sl[M_NPLANE * NPS];
+        angular_due();
         if constexpr (sizeof(R) == 4) {
             // event-major FP32 record (16-byte aligned): two values per load
             const float4* q4 = reinterpret_cast<const float4*>(slp);
@@ -493,14 +518,19 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
                 sl[c] = make_float2(x.x, x.y);
                 if (c + 1 < M_NPLANE * NPS) sl[c + 1] = make_float2(x.z, x.w);
             }
-        } else if constexpr (SL_EM) {
-            // event-major FP64 record: consecutive 16-byte values
+        } else if constexpr (SL_REAL) {
 #pragma unroll
-            for (int c = 0; c < M_NPLANE * NPS; ++c) sl[c] = slp[c];
+            for (int c = 0; c < M_NPLANE; ++c)
+#pragma unroll
+                for (int p = 0; p < NPS; ++p) {
+                    sl[c * NPS + p].x = slp[(long long)(c * M_NPOL + 2 * p) * ss];
+                    sl[c * NPS + p].y = 2 * p + 1 < M_NPOL ? slp[(long long)(c * M_NPOL + 2 * p + 1) * ss] : (R)0;
+                }
         } else {
 #pragma unroll
             for (int c = 0; c < M_NPLANE * NPS; ++c) sl[c] = slp[(long long)c * ss];
         }
+        angular_read();
         // c_t = v_col(t) F_t per term (one per column, more with identical particles)
         R cr[M_NTERM], ci[M_NTERM];
 #pragma unroll
@@ -546,8 +576,13 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
 #pragma unroll
                 for (int t = 0; t < M_NTERM; ++t) {
                     SL2 x = sl[term_plane(t) * NPS + p];
-                    sr += cr[t] * x.x - ci[t] * x.y;
-                    sim += cr[t] * x.y + ci[t] * x.x;
+                    if constexpr (SL_REAL) {  // (the polarisation paired with itself)
+                        sr += cr[t] * x.x;
+                        sim += ci[t] * x.x;
+                    } else {
+                        sr += cr[t] * x.x - ci[t] * x.y;
+                        sim += cr[t] * x.y + ci[t] * x.x;
+                    }
                 }
                 Sr[p] = sr;
                 Si[p] = sim;
@@ -613,8 +648,13 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
 #pragma unroll
             for (int p = 0; p < NPS; ++p) {
                 SL2 x = sl[c * NPS + p];
-                tr += x.x * ar[p] + x.y * br[p];
-                ti += x.x * ai[p] + x.y * bi[p];
+                if (SL_REAL && M_NPOL - 1 - p == p) {
+                    tr += x.x * ar[p];
+                    ti += x.x * ai[p];
+                } else {
+                    tr += x.x * ar[p] + x.y * br[p];
+                    ti += x.x * ai[p] + x.y * bi[p];
+                }
             }
             Tr[c] = tr;
             Ti[c] = ti;
@@ -654,7 +694,49 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
         ev.adjoint(sC, sCfh, sCfl, sink);
     };
 
-    if constexpr (STAGE == 3) {
+    auto nothing = [] {};
+    if constexpr (STAGE == 4) {
+        // Per-thread pipeline of the frontier and the angular values, one
+        // shared-memory slot per value and thread: a thread issues the copies
+        // of its next event's frontier values as soon as it has read the
+        // current ones into registers, and those of the angular values as
+        // soon as it has read these, so each copy has about one event's
+        // arithmetic to arrive and no second buffer is needed. At 12 warps
+        // per SM the FP64 kernel spent half of its cycles waiting for direct
+        // loads (K+K-pi0, 11.1M events 0.709 -> 0.561 ms with the table of
+        // reals, three chains of rho 5.55M 0.358 -> 0.287 ms).
+        // Copies are committed alternately (angular values of an event after
+        // its frontier values), so allowing one group in flight waits for the
+        // older of the two.
+        static_assert(sizeof(L) == 8 || STAGE != 4, "FP64 form");
+        constexpr int NA = M_NEV, NPL = SL_NPL;
+        SLT* sbuf = (SLT*)(ct_dyn + ACC_BYTES) + threadIdx.x;                                  // [NPL][BLOCK]
+        L* abuf = (L*)(ct_dyn + ACC_BYTES + (size_t)NPL * BLOCK * sizeof(SLT)) + threadIdx.x;  // [NA][BLOCK]
+        const long long stride = (long long)S.cta_count * BLOCK;
+        long long e = (long long)(cta - S.cta_begin) * BLOCK + threadIdx.x;
+        auto frontier = [&](long long x) {
+            if (x < n) {
+#pragma unroll
+                for (int k = 0; k < NA; ++k) ct_cp_async<8>(abuf + k * BLOCK, eva + (long long)k * S.ld + x);
+            }
+            ct_cp_async_commit();
+        };
+        auto angular = [&](long long x) {
+            if (x < n) {
+#pragma unroll
+                for (int c = 0; c < NPL; ++c) ct_cp_async<sizeof(SLT)>(sbuf + c * BLOCK, slamp + (long long)c * S.ld + x);
+            }
+            ct_cp_async_commit();
+        };
+        frontier(e);
+        angular(e);
+        for (; e < n; e += stride) {
+            ct_cp_async_wait<1>();
+            event(e, abuf, nullptr, BLOCK, sbuf, BLOCK, [&] { frontier(e + stride); }, [&] { ct_cp_async_wait<1>(); },
+                  [&] { angular(e + stride); });
+        }
+        ct_cp_async_wait<0>();
+    } else if constexpr (STAGE == 3) {
         // Per-thread two-buffer pipeline of the frontier values: each thread
         // copies its next event's frontier values into its own shared-memory
         // slots by cp.async while it computes the current event, and waits
@@ -691,7 +773,7 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
             else ct_cp_async_commit();  // empty group: the wait below covers buffer b alike
             ct_cp_async_wait<1>();
             const L* ap = CtEvent<L>::EVMAJ ? abuf + ((size_t)b * BLOCK + tid) * NA : abuf + (size_t)b * NA * BLOCK + tid;
-            event(e, ap, bbuf + (size_t)b * NB * BLOCK + tid, BLOCK, slat(e), S.ld);
+            event(e, ap, bbuf + (size_t)b * NB * BLOCK + tid, BLOCK, slat(e), S.ld, nothing, nothing, nothing);
         }
         ct_cp_async_wait<0>();
     } else if constexpr (STAGE > 0) {
@@ -703,10 +785,10 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
         // the current tile. No CTA-wide barrier: warps proceed independently.
         // Rows are padded to multiples of 256 events, so every copy starts on
         // a 128-byte boundary and moves a whole 32-event tile.
-        constexpr int NPL = M_NPLANE * (PAIRED ? CT_NPOL_STORED : M_NPOL);  // table rows
+        constexpr int NPL = SL_NPL;  // table rows
         constexpr int W = BLOCK / 32;
         constexpr int NA = CtEvent<L>::NA, NB = CtEvent<L>::NB;
-        constexpr unsigned AR = 32 * sizeof(L), BR = 32 * sizeof(double), SR = 32 * sizeof(SL2);
+        constexpr unsigned AR = 32 * sizeof(L), BR = 32 * sizeof(double), SR = 32 * sizeof(SLT);
         // angular part of a tile: NPL rows of 32 values (FP64), or 32 records of SL_SLS values (FP32)
         constexpr unsigned SLB = (SL_EM ? SL_SLS : NPL) * SR;
         constexpr unsigned BUF = NA * AR + NB * BR + (STAGE > 1 ? SLB : 0);
@@ -765,9 +847,10 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
                 const double* bp = (const double*)(buf + (size_t)NA * AR) + lane;
                 if constexpr (STAGE > 1)
                     event(e, ap, bp, 32,
-                          (const SL2*)(buf + (size_t)NA * AR + (size_t)NB * BR) + (SL_EM ? lane * SL_SLS : lane), 32);
+                          (const SLT*)(buf + (size_t)NA * AR + (size_t)NB * BR) + (SL_EM ? lane * SL_SLS : lane), 32,
+                          nothing, nothing, nothing);
                 else
-                    event(e, ap, bp, 32, slat(e), S.ld);
+                    event(e, ap, bp, 32, slat(e), S.ld, nothing, nothing, nothing);
             }
             // every lane is done with buffer b before it is refilled
             __syncwarp();
@@ -787,7 +870,7 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
     } else {
         const long long stride = (long long)S.cta_count * BLOCK;
         for (long long e = (long long)(cta - S.cta_begin) * BLOCK + threadIdx.x; e < n; e += stride)
-            event(e, CtEvent<L>::at(eva, e), evb ? evb + e : nullptr, S.ld, slat(e), S.ld);
+            event(e, CtEvent<L>::at(eva, e), evb ? evb + e : nullptr, S.ld, slat(e), S.ld, nothing, nothing, nothing);
     }
     ct_block_reduce_store<BLOCK, L>(accd, accg, A.partials + (long long)cta * CT_NACC, kind == 0 ? S.vw_scale : -1.0,
                                  kind == 0 ? 2.0 : -2.0, A.consts + M_NCONST);
@@ -813,7 +896,7 @@ extern "C" __global__ void __launch_bounds__(CT_F64_BLOCK, CT_F64_MINB) ct_fused
 }
 extern "C" __global__ void __launch_bounds__(CT_F64_BLOCK, CT_F64_MINB) ct_fused_f64_pc(CtArgs a)
 {
-    ct_fused_body<double, double, false, CT_F64_BLOCK, CT_F64_STAGE, CT_F64_ACC != 0, true>(a);
+    ct_fused_body<double, double, false, CT_F64_BLOCK, CT_F64_PC_STAGE, CT_F64_ACC != 0, true>(a);
 }
 // mixed form (FP32 lineshapes and algebra, FP64 logs and sums), all samples
 extern "C" __global__ void __launch_bounds__(CT_MX_BLOCK, CT_MX_MINB) ct_fused_mixed(CtArgs a)
@@ -844,7 +927,7 @@ extern "C" __global__ void __launch_bounds__(CT_F64_BLOCK, CT_F64_MINB)
 extern "C" __global__ void __launch_bounds__(CT_F64_BLOCK, CT_F64_MINB)
     ct_fused_f64_pc_multi(const CtArgs* __restrict__ jobs, const int* __restrict__ cta_off, int njobs)
 {
-    ct_fused_body<double, double, false, CT_F64_BLOCK, CT_F64_STAGE, CT_F64_ACC != 0, true, true>(
+    ct_fused_body<double, double, false, CT_F64_BLOCK, CT_F64_PC_STAGE, CT_F64_ACC != 0, true, true>(
         jobs[ct_multi_job(cta_off, njobs)]);
 }
 extern "C" __global__ void __launch_bounds__(CT_MX_BLOCK, CT_MX_MINB)

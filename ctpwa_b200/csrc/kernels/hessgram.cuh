@@ -41,6 +41,7 @@
 // throughout, so the sums are bit-reproducible.
 #pragma once
 
+#include "angular_load.cuh"
 #include "device_helpers.cuh"
 #include "model.cuh"
 #include "model_hess.cuh"
@@ -51,7 +52,7 @@
 #ifndef CT_HESS_MINB
 #define CT_HESS_MINB 2
 #endif
-// paired polarisations: compact event-major table (see hessian.cuh)
+// paired polarisations: table of reals (see hessian.cuh)
 #ifndef CT_HESS_PAIRED
 #define CT_HESS_PAIRED 0
 #endif
@@ -72,7 +73,7 @@ struct CtHessConsts {
 __constant__ CtHessConsts hs_k;
 
 struct CtHessSample {
-    const double2* slamp;  // [M_NPLANE * M_NPOL][ld]; paired: event-major [ld][M_NPLANE * stored]
+    const void* slamp;     // [M_NPLANE * M_NPOL][ld] angular values, complex, or real when paired
     const double* ev;      // [M_NEV][ld] FP64 frontier values
     const double* w;       // per-event weights or nullptr
     long long n;
@@ -406,9 +407,7 @@ extern "C" __global__ void __launch_bounds__(32 * CT_HESS_WARPS, CT_HESS_MINB) c
         double ev[M_NEV > 0 ? M_NEV : 1];
 #pragma unroll
         for (int k = 0; k < M_NEV; ++k) ev[k] = __ldg(S.ev + (long long)k * ld + e);
-#pragma unroll
-        for (int c = 0; c < M_NPLANE * CT_HNPS; ++c)
-            T.sl[c] = CT_HESS_PAIRED ? __ldg(S.slamp + e * (M_NPLANE * CT_HNPS) + c) : __ldg(S.slamp + (long long)c * ld + e);
+        ct_load_angular<CT_HESS_PAIRED != 0>(S.slamp, ld, e, T.sl);
         T.we = S.w ? __ldg(S.w + e) : 1.0;
         if (!T.active) T.we = 0.0;
         hs_columns(ev, hs_k.c, T);

@@ -24,6 +24,7 @@
 // phase-space weight total here (the finalize does it).
 #pragma once
 
+#include "angular_load.cuh"
 #include "device_helpers.cuh"
 #include "model.cuh"
 
@@ -103,7 +104,8 @@ __device__ __forceinline__ double ct_value(CtDual x) { return x.v; }
 #define CT_HVP_BLOCK 128
 #endif
 // paired polarisations (SL_{c,NPOL-1-p} = conj(SL_{c,p}) on every event): the
-// tables hold polarisations 0 .. (M_NPOL+1)/2 - 1 only, [plane][p][ld]
+// table holds M_NPOL reals per plane, [plane][x, y of each pair, one real for
+// the polarisation paired with itself][ld] (its constant phase drops out)
 #ifndef CT_HVP_PAIRED
 #define CT_HVP_PAIRED 0
 #endif
@@ -112,7 +114,7 @@ __device__ __forceinline__ double ct_value(CtDual x) { return x.v; }
 #define CT_HCONST_ALLOC (M_NCONST > 0 ? M_NCONST : 1)
 
 struct CtHvpSample {
-    const double2* slamp;  // [M_NPLANE * M_NPOL][ld] angular values; paired: event-major [ld][M_NPLANE * stored]
+    const void* slamp;     // [M_NPLANE * M_NPOL][ld] angular values, complex, or real when paired
     const double* ev;      // [M_NEV][ld] FP64 frontier values
     const double* w;       // per-event weights or nullptr
     long long n;
@@ -220,10 +222,7 @@ extern "C" __global__ void __launch_bounds__(CT_HVP_BLOCK) ct_hvp_f64(CtHvpArgs 
             else model_columns(ev, sCv, Fr, Fi, dFr, dFi);
             constexpr int NPS = CT_HVP_PAIRED ? (M_NPOL + 1) / 2 : M_NPOL;
             double2 sl[M_NPLANE * NPS];
-#pragma unroll
-            for (int c = 0; c < M_NPLANE * NPS; ++c)
-                sl[c] = CT_HVP_PAIRED ? __ldg(S.slamp + e * (M_NPLANE * NPS) + c)  // compact table: event-major
-                                      : __ldg(S.slamp + (long long)c * ld + e);
+            ct_load_angular<CT_HVP_PAIRED != 0>(S.slamp, ld, e, sl);
             CtDual cr[M_NTERM], ci[M_NTERM];
 #pragma unroll
             for (int t = 0; t < M_NTERM; ++t) {
