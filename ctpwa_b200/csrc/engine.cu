@@ -1911,7 +1911,13 @@ FusedShape fusedShape(const GeneratedModel& gen)
         if (v < lo || v > hi) throw std::runtime_error(std::string(name) + " out of range");
         return v;
     };
-    sh.block[0] = get("CTPWA_F64_BLOCK", 192, 32, 1024);
+    // plain path: 256 threads where the sums and the copies of paired
+    // polarisations fit twice per SM (16 warps, at 128 registers), else 192
+    // (12 warps): three chains of rho 5.55M events 0.262 ms against 0.287 ms,
+    // K_S K_S 1.1M events 0.045 against 0.047 ms; K+K-pi0 has room for 192
+    // only (256 with direct loads 0.61 ms against 0.56 ms)
+    const long long f64_bytes = (gen.nsum[0] + (long long)std::max(1, gen.nplane) * std::max(1, gen.npol) + gen.nev64) * 8;
+    sh.block[0] = get("CTPWA_F64_BLOCK", 2 * (f64_bytes * 256 + 8 * 1024) <= 228 * 1024 ? 256 : 192, 32, 1024);
     sh.minb[0] = get("CTPWA_F64_MINB", 2, 1, 16);
     sh.block[1] = get("CTPWA_MX_BLOCK", 256, 32, 1024);
     sh.minb[1] = get("CTPWA_MX_MINB", 2, 1, 16);
@@ -2119,7 +2125,7 @@ HessShape hessShape(const GeneratedModel& gen)
     if (gen.hess_header.empty() || hp < 1 || hb > 6) return h;
     h.blocks = hb;
     h.row = hb * (hb + 1) / 2 * 64 + gen.nhlin + 1;
-    const int slab = std::max(std::max(8 * hb * 68, 32 * 33), h.row);
+    const int slab = std::max(std::max(8 * hb * 68, 32 * 33) + 68, h.row);  // CT_HSLAB, reused for the CTA's row
     h.dsmem = h.warps * slab * (int)sizeof(double);
     if (h.dsmem > 110 * 1024) h.minb = 1;
     if (h.dsmem > 220 * 1024) h.blocks = 0;
@@ -3147,10 +3153,10 @@ void Engine::compileHess()
 }
 
 // The one-pass form costs the same for any number of directions, forward mode
-// a pass per direction: K+K-pi0, 11.1M events, 5.4 ms against 1.3 ms per
-// direction (30.1 ms for all 23); three chains of rho, 1.11M events, 0.62 ms
+// a pass per direction: K+K-pi0, 11.1M events, 4.0 ms against 1.3 ms per
+// direction (30.1 ms for all 23); three chains of rho, 1.11M events, 0.51 ms
 // against 0.13 ms (3.2 ms for all 24).
-bool Engine::onePassHessian(int ndir) const { return ndir >= 5 && hessShape(gen_).blocks > 0; }
+bool Engine::onePassHessian(int ndir) const { return ndir >= 4 && hessShape(gen_).blocks > 0; }
 
 // The one pass over the events and the contraction with the directions; the
 // value sums of the same pass too when d_vsums is given. d_v_ holds the couplings.

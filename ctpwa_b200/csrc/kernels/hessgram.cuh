@@ -28,9 +28,11 @@
 // amplitudes in dual numbers for each of the nparam directions; here they are
 // computed once. Per 32 K+K-pi0 events (HP = 23, 3 polarisations) 288 block
 // products (336 with the rank-one term), 16 cycles each on a quarter of an
-// SM, and ~1760 other FP64 instructions, 2 cycles each: bound by the FP64
+// SM, and ~1600 other FP64 instructions, 2 cycles each: bound by the FP64
 // pipe and, at 8 warps per SM (255 registers), by its latency. 11.1M events:
-// 30.1 -> 5.4 ms; three chains of rho, 1.11M events: 3.22 -> 0.62 ms.
+// 30.1 -> 4.0 ms; three chains of rho, 1.11M events: 3.22 -> 0.51 ms (5.4 and
+// 0.62 ms with signs and row ends tested in every k-step and four products
+// per term and polarisation).
 //
 // Clamps as in the gradient pass: components of w S / f beyond 1e10 count as
 // constants (no derivative). Only then are the weights of a polarisation's
@@ -65,6 +67,10 @@
 // of a fragment read fall in different banks
 #define CT_HRS 68
 #define CT_HNPS (CT_HESS_PAIRED ? (M_NPOL + 1) / 2 : M_NPOL)
+// a warp's slab: the rows of the matrix (the linear sums' [32][33] use its
+// start), then one row of zeros that the lanes of the rows past CT_HP read
+#define CT_HROWS (8 * CT_HB * CT_HRS > 32 * 33 ? 8 * CT_HB * CT_HRS : 32 * 33)
+#define CT_HSLAB (CT_HROWS + CT_HRS)
 
 struct CtHessConsts {
     double c[M_NHC > 0 ? M_NHC : 1];
@@ -111,7 +117,7 @@ __device__ __forceinline__ void ct_dmma(double (&c)[2], double a, double b)
 // One warp's working state for a tile of 32 events (one per lane): the sink
 // of hs_columns.
 struct CtHessTile {
-    double* slab;   // [8 * CT_HB][CT_HRS] (and [32][33] for the linear sums)
+    double* slab;   // [CT_HSLAB]
     int lane;
     // per event
     double Fr[M_NTERM], Fi[M_NTERM];
@@ -138,6 +144,8 @@ struct CtHessTile {
         const double2 x = sl[c * CT_HNPS + q];
         return make_double2(x.x, -x.y);
     }
+    // the polarisation paired with itself: real angular values
+    static __device__ __forceinline__ constexpr bool realPol(int p) { return CT_HESS_PAIRED && M_NPOL - 1 - p == p; }
     __device__ __forceinline__ void value(int t, double re, double im)
     {
         Fr[t] = re;
@@ -146,18 +154,33 @@ struct CtHessTile {
     // coherent sums, event weight, contraction of the angular values
     __device__ __forceinline__ void sums()
     {
-        double Sr[M_NPOL], Si[M_NPOL];
+        double Sr[M_NPOL], Si[M_NPOL], xr[M_NPOL], yi[M_NPOL], yr[M_NPOL], xi[M_NPOL];
 #pragma unroll
-        for (int p = 0; p < M_NPOL; ++p) Sr[p] = Si[p] = 0.0;
+        for (int p = 0; p < M_NPOL; ++p) xr[p] = yi[p] = yr[p] = xi[p] = 0.0;
 #pragma unroll
         for (int t = 0; t < M_NTERM; ++t) {
             const double vr = hs_k.v[2 * term_col(t)], vi = hs_k.v[2 * term_col(t) + 1];
             const double tr = vr * Fr[t] - vi * Fi[t], ti = vr * Fi[t] + vi * Fr[t];
 #pragma unroll
-            for (int p = 0; p < M_NPOL; ++p) {
-                const double2 x = pol(term_plane(t), p);
-                Sr[p] += tr * x.x - ti * x.y;
-                Si[p] += tr * x.y + ti * x.x;
+            for (int p = 0; p < CT_HNPS; ++p) {
+                const double2 x = sl[term_plane(t) * CT_HNPS + p];
+                xr[p] += tr * x.x;
+                xi[p] += ti * x.x;
+                if (!realPol(p)) {
+                    yr[p] += tr * x.y;
+                    yi[p] += ti * x.y;
+                }
+            }
+        }
+        // S_p = sum c (x + iy); paired: S_q = sum c (x - iy) from the same products
+#pragma unroll
+        for (int p = 0; p < CT_HNPS; ++p) {
+            const int q = M_NPOL - 1 - p;
+            Sr[p] = realPol(p) ? xr[p] : xr[p] - yi[p];
+            Si[p] = realPol(p) ? xi[p] : xi[p] + yr[p];
+            if (CT_HESS_PAIRED && q != p) {
+                Sr[q] = xr[p] + yi[p];
+                Si[q] = xi[p] - yr[p];
             }
         }
         double ur[M_NPOL], ui[M_NPOL];
@@ -210,10 +233,20 @@ struct CtHessTile {
         for (int c = 0; c < M_NPLANE; ++c) {
             double x = 0.0, y = 0.0;
 #pragma unroll
-            for (int p = 0; p < M_NPOL; ++p) {
-                const double2 s = pol(c, p);
-                x += s.x * ur[p] + s.y * ui[p];
-                y += s.y * ur[p] - s.x * ui[p];
+            for (int p = 0; p < CT_HNPS; ++p) {
+                const int q = M_NPOL - 1 - p;
+                const double2 s = sl[c * CT_HNPS + p];
+                if (realPol(p)) {
+                    x += s.x * ur[p];
+                    y -= s.x * ui[p];
+                } else if (CT_HESS_PAIRED) {
+                    // SL_p conj(u_p) + conj(SL_p) conj(u_q)
+                    x += s.x * (ur[p] + ur[q]) + s.y * (ui[p] - ui[q]);
+                    y += s.y * (ur[p] - ur[q]) - s.x * (ui[p] + ui[q]);
+                } else {
+                    x += s.x * ur[p] + s.y * ui[p];
+                    y += s.y * ur[p] - s.x * ui[p];
+                }
             }
             o_r[c] = x;
             o_i[c] = y;
@@ -254,25 +287,25 @@ struct CtHessTile {
         put(r, 2.0 * (re * wr - im * wi));
     }
     // the symmetric update by the slab's KS k-steps of 4 columns (LOGE: log2
-    // of the columns per event); neg: lanes whose event enters with a minus
-    template <int KS, int LOGE>
+    // of the columns per event). SIGN 0: added, 1: subtracted, 2: subtracted
+    // for the events of the lanes in `neg`, added for the others
+    template <int KS, int LOGE, int SIGN>
     __device__ __forceinline__ void update(unsigned neg)
     {
         __syncwarp();
         const double* base = slab + (lane >> 2) * CT_HRS + (lane & 3);
+        const double* last = 8 * (CT_HB - 1) + (lane >> 2) < CT_HP ? base + (CT_HB - 1) * 8 * CT_HRS
+                                                                    : slab + CT_HROWS + (lane & 3);
 #pragma unroll 4
         for (int s = 0; s < KS; ++s) {
             double b[CT_HB];
 #pragma unroll
-            for (int I = 0; I < CT_HB; ++I) {
-                b[I] = base[I * 8 * CT_HRS + 4 * s];
-                if (8 * I + 7 >= CT_HP && 8 * I + (lane >> 2) >= CT_HP) b[I] = 0.0;
-            }
-            const bool minus = neg != 0 && ((neg >> ((4 * s + (lane & 3)) >> LOGE)) & 1u);
+            for (int I = 0; I < CT_HB; ++I) b[I] = I + 1 < CT_HB ? base[I * 8 * CT_HRS + 4 * s] : last[4 * s];
+            const bool minus = SIGN == 2 && ((neg >> ((4 * s + (lane & 3)) >> LOGE)) & 1u);
             int q = 0;
 #pragma unroll
             for (int I = 0; I < CT_HB; ++I) {
-                const double a = minus ? -b[I] : b[I];
+                const double a = SIGN == 1 || (SIGN == 2 && minus) ? -b[I] : b[I];
 #pragma unroll
                 for (int J = I; J < CT_HB; ++J) ct_dmma(acc[q++], a, b[J]);
             }
@@ -308,48 +341,65 @@ struct CtHessTile {
                 }
             o[(2 * M_NA + j) * CT_HRS] = scale * g;
         }
-        update<8, 0>(__ballot_sync(0xffffffffu, (we > 0.0) != flip));
+        // (rows of weight zero are zero, whatever their sign)
+        const unsigned neg = __ballot_sync(0xffffffffu, we != 0.0 && (we > 0.0) != flip);
+        const unsigned pos = __ballot_sync(0xffffffffu, we != 0.0 && (we > 0.0) == flip);
+        if (pos == 0) update<8, 0, 1>(0);
+        else update<8, 0, 2>(neg);
+    }
+    // (xr, xi) += (fr + i fi) SL_{c,p}
+    __device__ __forceinline__ void addProduct(double& xr, double& xi, double fr, double fi, int c, int p) const
+    {
+        const double2 s = pol(c, p);
+        if (realPol(p)) {
+            xr += fr * s.x;
+            xi += fi * s.x;
+        } else {
+            xr += fr * s.x - fi * s.y;
+            xi += fr * s.y + fi * s.x;
+        }
     }
     __device__ __forceinline__ void finish()
     {
         if (M_HLIN % 32) flush(M_HLIN / 32, M_HLIN % 32);
-        // polarisations: rows sqrt(2 |alpha|) d_i S_p
+        // polarisations: rows sqrt(2 |alpha|) d_i S_p (the factor on the angular values)
         const double sg = sqrt(2.0 * fabs(alpha));
         const unsigned neg = __ballot_sync(0xffffffffu, alpha < 0.0);
 #pragma unroll
+        for (int c = 0; c < M_NPLANE * CT_HNPS; ++c) {
+            sl[c].x *= sg;
+            if (!realPol(c % CT_HNPS)) sl[c].y *= sg;
+        }
+#pragma unroll
         for (int p = 0; p < M_NPOL; ++p) {
-            double kr = sg, ki = sg;
-            if (any) {
-                if ((mask >> (2 * p)) & 1) kr = 0.0;
-                if ((mask >> (2 * p)) & 2) ki = 0.0;
-            }
             double2* o = reinterpret_cast<double2*>(slab) + lane;
 #pragma unroll
             for (int a = 0; a < M_NA; ++a) {
                 double xr = 0.0, xi = 0.0;
 #pragma unroll
                 for (int t = 0; t < M_NTERM; ++t)
-                    if (term_col(t) == a) {
-                        const double2 s = pol(term_plane(t), p);
-                        xr += Fr[t] * s.x - Fi[t] * s.y;
-                        xi += Fr[t] * s.y + Fi[t] * s.x;
-                    }
-                o[a * (CT_HRS / 2)] = make_double2(kr * xr, ki * xi);
-                o[(M_NA + a) * (CT_HRS / 2)] = make_double2(-kr * xi, ki * xr);
+                    if (term_col(t) == a) addProduct(xr, xi, Fr[t], Fi[t], term_plane(t), p);
+                o[a * (CT_HRS / 2)] = make_double2(xr, xi);
+                o[(M_NA + a) * (CT_HRS / 2)] = make_double2(-xi, xr);
             }
 #pragma unroll
             for (int j = 0; j < M_NTH; ++j) {
                 double xr = 0.0, xi = 0.0;
 #pragma unroll
                 for (int k = 0; k < M_NDER; ++k)
-                    if (der_th(k) == j) {
-                        const double2 s = pol(term_plane(der_term(k)), p);
-                        xr += Wr[k] * s.x - Wi[k] * s.y;
-                        xi += Wr[k] * s.y + Wi[k] * s.x;
-                    }
-                o[(2 * M_NA + j) * (CT_HRS / 2)] = make_double2(kr * xr, ki * xi);
+                    if (der_th(k) == j) addProduct(xr, xi, Wr[k], Wi[k], term_plane(der_term(k)), p);
+                o[(2 * M_NA + j) * (CT_HRS / 2)] = make_double2(xr, xi);
             }
-            update<16, 1>(neg);
+            // clamped components drop out
+            if (any) {
+#pragma unroll 1
+                for (int i = 0; i < CT_HP; ++i) {
+                    if ((mask >> (2 * p)) & 1) slab[i * CT_HRS + 2 * lane] = 0.0;
+                    if ((mask >> (2 * p)) & 2) slab[i * CT_HRS + 2 * lane + 1] = 0.0;
+                }
+            }
+            if (neg == 0) update<16, 1, 0>(0);
+            else update<16, 1, 2>(neg);
         }
         if (kind != 0) {
             const double rs = we != 0.0 ? 1.0 / sqrt(fabs(we)) : 0.0;
@@ -381,7 +431,6 @@ struct CtHessTile {
 
 extern "C" __global__ void __launch_bounds__(32 * CT_HESS_WARPS, CT_HESS_MINB) ct_hess_f64(CtHessArgs A)
 {
-    constexpr int SLAB = 8 * CT_HB * CT_HRS > 32 * 33 ? 8 * CT_HB * CT_HRS : 32 * 33;
     extern __shared__ __align__(16) double ct_hs[];
     const int cta = (int)blockIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     int si = 0;
@@ -390,7 +439,8 @@ extern "C" __global__ void __launch_bounds__(32 * CT_HESS_WARPS, CT_HESS_MINB) c
         if (k < A.nsamp && cta >= A.s[k].cta_begin) si = k;
     const CtHessSample& S = A.s[si];
     CtHessTile T;
-    T.slab = ct_hs + warp * SLAB;
+    T.slab = ct_hs + warp * CT_HSLAB;
+    for (int i = lane; i < CT_HRS; i += 32) T.slab[CT_HROWS + i] = 0.0;
     T.lane = lane;
     T.kind = S.kind;
     T.nlog = 0.0;
