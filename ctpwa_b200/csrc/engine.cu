@@ -1413,20 +1413,20 @@ std::string angularSource(const std::vector<AgGroupHost>& gh, const std::vector<
             }
             if (npair > 0) {
                 for (int p = 0; p < A.npol; ++p)
-                    o << "    big = fmax(big, agDist(c" << last << "[" << srcs[p] << "].x, c" << last << "[" << srcs[p]
+                    o << "    big = fmax(big, agDist2(c" << last << "[" << srcs[p] << "].x, c" << last << "[" << srcs[p]
                       << "].y));\n";
                 if (A.npol % 2) {
                     const std::string c = "c" + std::to_string(last) + "[" + std::to_string(srcs[npair]) + "]";
-                    o << "    mid[0] = fmax(mid[0], agDist(" << c << ".x, 0.0)); mid[1] = fmax(mid[1], agDist(" << c
+                    o << "    mid[0] = fmax(mid[0], agDist2(" << c << ".x, 0.0)); mid[1] = fmax(mid[1], agDist2(" << c
                       << ".y, 0.0));\n";
                 }
                 for (int q = 0; q < npair; ++q) {
                     const std::string a = "c" + std::to_string(last) + "[" + std::to_string(srcs[q]) + "]",
                                       b = "c" + std::to_string(last) + "[" + std::to_string(srcs[A.npol - 1 - q]) + "]";
                     const int k = (s * npair + q) * 2;
-                    o << "    pm[" << k << "] = fmax(pm[" << k << "], agDist(" << b << ".x - " << a << ".x, " << b << ".y + "
+                    o << "    pm[" << k << "] = fmax(pm[" << k << "], agDist2(" << b << ".x - " << a << ".x, " << b << ".y + "
                       << a << ".y));\n";
-                    o << "    pm[" << k + 1 << "] = fmax(pm[" << k + 1 << "], agDist(" << b << ".x + " << a << ".x, " << b
+                    o << "    pm[" << k + 1 << "] = fmax(pm[" << k + 1 << "], agDist2(" << b << ".x + " << a << ".x, " << b
                       << ".y - " << a << ".y));\n";
                 }
             }
@@ -1440,12 +1440,12 @@ std::string angularSource(const std::vector<AgGroupHost>& gh, const std::vector<
                     for (int w = 0; w < 2; ++w) {
                         const int k = (s * npair + q) * 2 + w;
                         const int out = ((A.plane0 + s) * npair + q) * 2 + w;
-                        o << "    { const double v = agWarpMax(pm[" << k << "]); if (lane == 0) atomicMax(pairmax + " << out
+                        o << "    { const double v = sqrt(agWarpMax(pm[" << k << "])); if (lane == 0) atomicMax(pairmax + " << out
                           << ", (unsigned long long)__double_as_longlong(v)); }\n";
                     }
             for (int w = 0; w < 3; ++w)
-                o << "    { const double v = agWarpMax(" << (w == 0 ? "big" : w == 1 ? "mid[0]" : "mid[1]")
-                  << "); if (lane == 0) atomicMax(pairmax + " << 2 * nplane * npair + w
+                o << "    { const double v = sqrt(agWarpMax(" << (w == 0 ? "big" : w == 1 ? "mid[0]" : "mid[1]")
+                  << ")); if (lane == 0) atomicMax(pairmax + " << 2 * nplane * npair + w
                   << ", (unsigned long long)__double_as_longlong(v)); }\n";
             o << "  }\n";
         }
