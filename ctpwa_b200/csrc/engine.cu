@@ -3562,7 +3562,7 @@ void Engine::hessianGram(const double* d_params, double* d_hess, cudaStream_t st
         CT_CUDA(cudaMallocAsync((void**)&d_dirs, sizeof(double) * dirs.size(), stream));
         CT_CUDA(cudaMallocAsync((void**)&d_rows, sizeof(double) * dirs.size(), stream));
         CT_CUDA(cudaMemcpyAsync(d_dirs, dirs.data(), sizeof(double) * dirs.size(), cudaMemcpyHostToDevice, stream));
-        hessianVectorProducts(d_params, d_dirs, nT, d_rows, stream);
+        hessianRows(d_params, d_dirs, nT, d_rows, stream);
         std::vector<double> rows(dirs.size());
         CT_CUDA(cudaMemcpyAsync(rows.data(), d_rows, sizeof(double) * rows.size(), cudaMemcpyDeviceToHost, stream));
         CT_CUDA(cudaFreeAsync(d_dirs, stream));
@@ -3852,19 +3852,26 @@ void Engine::hessianVectorProducts(const double* d_params, const double* d_dirs,
     }
 }
 
+// Rows H u of up to hvp_cap_ directions, by whichever form is faster.
+void Engine::hessianRows(const double* d_params, const double* d_dirs, int ndir, double* d_out, cudaStream_t stream)
+{
+    if (!onePassHessian(ndir)) {
+        hessianVectorProducts(d_params, d_dirs, ndir, d_out, stream);
+        return;
+    }
+    const int nA = model_.nAmp();
+    ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, model_.nVector(), d_v_,
+                                                            d_err_);
+    CT_CUDA(cudaGetLastError());
+    hessSums(d_params, d_dirs, ndir, d_htsums_, d_hvsums_, stream);
+    finalizeHvp(d_params, d_dirs, ndir, d_hvsums_, d_htsums_, d_out, stream);
+}
+
 void Engine::hessianExact(const double* d_params, double* d_hess, cudaStream_t stream)
 {
     hvpBuffers();
-    const int n = model_.nParams(), nA = model_.nAmp();
-    if (onePassHessian(n)) {
-        ct_prepare_kernel<<<(nA + 127) / 128, 128, 0, stream>>>(d_params, d_amp_chain_, d_ratio_, nA, model_.nVector(),
-                                                                d_v_, d_err_);
-        CT_CUDA(cudaGetLastError());
-        hessSums(d_params, d_hdirs_, n, d_htsums_, d_hvsums_, stream);
-        finalizeHvp(d_params, d_hdirs_, n, d_hvsums_, d_htsums_, d_hess, stream);
-    } else {
-        hessianVectorProducts(d_params, d_hdirs_, n, d_hess, stream);
-    }
+    const int n = model_.nParams();
+    hessianRows(d_params, d_hdirs_, n, d_hess, stream);
     ct_symmetrize_kernel<<<std::max(1, (n * n + 255) / 256), 256, 0, stream>>>(d_hess, n);
     CT_CUDA(cudaGetLastError());
 }

@@ -244,6 +244,7 @@ private:
     // one-pass Hessian sums (kernels/hessgram.cuh; compiled and allocated on first use)
     void compileHess();
     bool onePassHessian(int ndir) const;
+    void hessianRows(const double* d_params, const double* d_dirs, int ndir, double* d_out, cudaStream_t stream);
     void hessSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums, double* d_vsums,
                   cudaStream_t stream);
     void* k_hess_pro_ = nullptr;
