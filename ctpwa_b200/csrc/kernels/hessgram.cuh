@@ -30,9 +30,10 @@
 // products (336 with the rank-one term), 16 cycles each on a quarter of an
 // SM, and ~1600 other FP64 instructions, 2 cycles each: bound by the FP64
 // pipe and, at 8 warps per SM (255 registers), by its latency. 11.1M events:
-// 30.1 -> 4.0 ms; three chains of rho, 1.11M events: 3.22 -> 0.51 ms (5.4 and
+// 30.1 -> 3.8 ms; three chains of rho, 1.11M events: 3.22 -> 0.48 ms (5.4 and
 // 0.62 ms with signs and row ends tested in every k-step and four products
-// per term and polarisation).
+// per term and polarisation; 3.95 and 0.51 ms with the rank-one term after the
+// polarisations', which keeps its plane sums in registers through them).
 //
 // Clamps as in the gradient pass: components of w S / f beyond 1e10 count as
 // constants (no derivative). Only then are the weights of a polarisation's
@@ -124,8 +125,6 @@ struct CtHessTile {
     double Wr[M_NDER > 0 ? M_NDER : 1], Wi[M_NDER > 0 ? M_NDER : 1];  // v dF_k
     double2 sl[M_NPLANE * CT_HNPS];
     double cr[M_NPLANE], ci[M_NPLANE];  // sum_p SL_{c,p} conj(u_p), u the clamped w S / f
-    double ar[M_NPLANE], ai[M_NPLANE];  // the same from unclamped and from unmasked components (clamped tiles only)
-    double yr[M_NPLANE], yi[M_NPLANE];
     double we, alpha, nlog;
     unsigned mask;  // clamped components, 2 p + (0 re, 1 im)
     bool any;       // some lane of the warp clamps
@@ -151,10 +150,10 @@ struct CtHessTile {
         Fr[t] = re;
         Fi[t] = im;
     }
-    // coherent sums, event weight, contraction of the angular values
-    __device__ __forceinline__ void sums()
+    // coherent sums S_p
+    __device__ __forceinline__ void coherent(double* Sr, double* Si) const
     {
-        double Sr[M_NPOL], Si[M_NPOL], xr[M_NPOL], yi[M_NPOL], yr[M_NPOL], xi[M_NPOL];
+        double xr[M_NPOL], yi[M_NPOL], yr[M_NPOL], xi[M_NPOL];
 #pragma unroll
         for (int p = 0; p < M_NPOL; ++p) xr[p] = yi[p] = yr[p] = xi[p] = 0.0;
 #pragma unroll
@@ -183,40 +182,38 @@ struct CtHessTile {
                 Si[q] = xi[p] - yr[p];
             }
         }
+    }
+    // coherent sums, event weight, contraction of the angular values
+    __device__ __forceinline__ void sums()
+    {
         double ur[M_NPOL], ui[M_NPOL];
+        coherent(ur, ui);
         mask = 0;
         if (kind == 0) {
             alpha = active ? we : 0.0;
 #pragma unroll
             for (int p = 0; p < M_NPOL; ++p) {
-                ur[p] = alpha * Sr[p];
-                ui[p] = alpha * Si[p];
+                ur[p] *= alpha;
+                ui[p] *= alpha;
             }
         } else {
             double f = 0.0;
 #pragma unroll
-            for (int p = 0; p < M_NPOL; ++p) f += Sr[p] * Sr[p] + Si[p] * Si[p];
+            for (int p = 0; p < M_NPOL; ++p) f += ur[p] * ur[p] + ui[p] * ui[p];
             // f == 0: the constant -w log(1e-10), no derivative
             if (active) nlog += f == 0.0 ? -log(1e-10) * we : -log(f) * we;
             alpha = active && f != 0.0 ? we / f : 0.0;
+            // (a NaN, 0 times an overflowed w / f, clamps as in forward mode)
 #pragma unroll
             for (int p = 0; p < M_NPOL; ++p) {
-                ur[p] = alpha * Sr[p];
-                ui[p] = alpha * Si[p];
-                if (fabs(ur[p]) > 1e10) mask |= 1u << (2 * p);
-                if (fabs(ui[p]) > 1e10) mask |= 2u << (2 * p);
+                ur[p] *= alpha;
+                ui[p] *= alpha;
+                if (!(fabs(ur[p]) <= 1e10)) mask |= 1u << (2 * p);
+                if (!(fabs(ui[p]) <= 1e10)) mask |= 2u << (2 * p);
             }
         }
         any = __any_sync(0xffffffffu, mask != 0);
         if (any) {
-            contract(ur, ui, yr, yi);
-            double mr[M_NPOL], mi[M_NPOL];
-#pragma unroll
-            for (int p = 0; p < M_NPOL; ++p) {
-                mr[p] = (mask >> (2 * p)) & 1 ? 0.0 : ur[p];
-                mi[p] = (mask >> (2 * p)) & 2 ? 0.0 : ui[p];
-            }
-            contract(mr, mi, ar, ai);
 #pragma unroll
             for (int p = 0; p < M_NPOL; ++p) {
                 ur[p] = fmin(fmax(ur[p], -1e10), 1e10);
@@ -313,9 +310,10 @@ struct CtHessTile {
         __syncwarp();
     }
     // rank-one update by the gradient rows of the plane vector (pr, pi):
-    // minus its square over w (sign: minus it for the difference vector of a clamped tile)
-    __device__ __forceinline__ void rank1(const double* pr, const double* pi, double scale, bool flip)
+    // minus its square over w (flip: plus)
+    __device__ __forceinline__ void rank1(const double* pr, const double* pi, bool flip)
     {
+        const double scale = we != 0.0 ? 1.0 / sqrt(fabs(we)) : 0.0;
         double* o = slab + lane;
 #pragma unroll
         for (int a = 0; a < M_NA; ++a) {
@@ -347,6 +345,47 @@ struct CtHessTile {
         if (pos == 0) update<8, 0, 1>(0);
         else update<8, 0, 2>(neg);
     }
+    // The plane vectors of a tile with clamps. With y the contraction of all
+    // unclamped components w S / f and a that of the components that are not
+    // clamped, the rank-one term is minus a y^T / w, symmetrised:
+    // (a y^T + y a^T) / 2 = ((a + y)(a + y)^T - (a - y)(a - y)^T) / 4. Both are
+    // scaled to the same size first, which leaves their product as it is: y
+    // may be 1e10 times a and more, and its square would drown the sums of all
+    // other events in rounding. Rare, so the coherent sums are formed again and
+    // nothing of this is kept through the derivatives.
+    __device__ __forceinline__ void clampedVectors(double* ar, double* ai, double* yr, double* yi) const
+    {
+        double ur[M_NPOL], ui[M_NPOL];
+        coherent(ur, ui);
+#pragma unroll
+        for (int p = 0; p < M_NPOL; ++p) {
+            ur[p] *= alpha;
+            ui[p] *= alpha;
+        }
+        contract(ur, ui, yr, yi);
+#pragma unroll
+        for (int p = 0; p < M_NPOL; ++p) {
+            if ((mask >> (2 * p)) & 1) ur[p] = 0.0;
+            if ((mask >> (2 * p)) & 2) ui[p] = 0.0;
+        }
+        contract(ur, ui, ar, ai);
+        double na = 0.0, ny = 0.0;
+#pragma unroll
+        for (int c = 0; c < M_NPLANE; ++c) {
+            na = fmax(na, fmax(fabs(ar[c]), fabs(ai[c])));
+            ny = fmax(ny, fmax(fabs(yr[c]), fabs(yi[c])));
+        }
+        // (all components clamped: a is zero, y possibly infinite)
+        const bool none = !(na > 0.0 && ny > 0.0);
+        const double sy = none ? 0.0 : sqrt(na / ny), sa = none ? 0.0 : sqrt(ny / na);
+#pragma unroll
+        for (int c = 0; c < M_NPLANE; ++c) {
+            ar[c] *= sa;
+            ai[c] *= sa;
+            yr[c] = none ? 0.0 : yr[c] * sy;
+            yi[c] = none ? 0.0 : yi[c] * sy;
+        }
+    }
     // (xr, xi) += (fr + i fi) SL_{c,p}
     __device__ __forceinline__ void addProduct(double& xr, double& xi, double fr, double fi, int c, int p) const
     {
@@ -362,6 +401,30 @@ struct CtHessTile {
     __device__ __forceinline__ void finish()
     {
         if (M_HLIN % 32) flush(M_HLIN / 32, M_HLIN % 32);
+        if (kind != 0) {
+            // g = (w / f) grad f, the term -(w / f^2) grad f grad f^T = -g g^T / w
+            double pr[M_NPLANE], pi[M_NPLANE];
+            if (!any) {
+#pragma unroll
+                for (int c = 0; c < M_NPLANE; ++c) {
+                    pr[c] = 2.0 * cr[c];
+                    pi[c] = 2.0 * ci[c];
+                }
+                rank1(pr, pi, false);
+            } else {
+                double ar[M_NPLANE], ai[M_NPLANE], yr[M_NPLANE], yi[M_NPLANE];
+                clampedVectors(ar, ai, yr, yi);
+#pragma unroll 1
+                for (int h = 0; h < 2; ++h) {
+#pragma unroll
+                    for (int c = 0; c < M_NPLANE; ++c) {
+                        pr[c] = ar[c] + (h ? -yr[c] : yr[c]);
+                        pi[c] = ai[c] + (h ? -yi[c] : yi[c]);
+                    }
+                    rank1(pr, pi, h != 0);
+                }
+            }
+        }
         // polarisations: rows sqrt(2 |alpha|) d_i S_p (the factor on the angular values)
         const double sg = sqrt(2.0 * fabs(alpha));
         const unsigned neg = __ballot_sync(0xffffffffu, alpha < 0.0);
@@ -400,31 +463,6 @@ struct CtHessTile {
             }
             if (neg == 0) update<16, 1, 0>(0);
             else update<16, 1, 2>(neg);
-        }
-        if (kind != 0) {
-            const double rs = we != 0.0 ? 1.0 / sqrt(fabs(we)) : 0.0;
-            if (!any) {
-                // g = (w / f) grad f, the term -(w / f^2) grad f grad f^T = -g g^T / w
-                double pr[M_NPLANE], pi[M_NPLANE];
-#pragma unroll
-                for (int c = 0; c < M_NPLANE; ++c) {
-                    pr[c] = 2.0 * cr[c];
-                    pi[c] = 2.0 * ci[c];
-                }
-                rank1(pr, pi, rs, false);
-            } else {
-                // (a y^T + y a^T) / 2 = ((a + y)(a + y)^T - (a - y)(a - y)^T) / 4
-#pragma unroll 1
-                for (int h = 0; h < 2; ++h) {
-                    double pr[M_NPLANE], pi[M_NPLANE];
-#pragma unroll
-                    for (int c = 0; c < M_NPLANE; ++c) {
-                        pr[c] = ar[c] + (h ? -yr[c] : yr[c]);
-                        pi[c] = ai[c] + (h ? -yi[c] : yi[c]);
-                    }
-                    rank1(pr, pi, rs, h != 0);
-                }
-            }
         }
     }
 };

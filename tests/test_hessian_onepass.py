@@ -22,7 +22,8 @@ def _many_resonances(nres):
         for i, n in enumerate(names))
 
 
-def _compare(tmp_path, text, masses, sizes, weights=(False, False, False), seed=1):
+def _setup(tmp_path, text, masses, sizes, weights=(False, False, False), seed=1, few=()):
+    """An analysis over phase-space samples, and its parameters. few: weights of the first data events."""
     import torch
 
     import ctpwa_b200
@@ -37,15 +38,27 @@ def _compare(tmp_path, text, masses, sizes, weights=(False, False, False), seed=
     # signed weights: data and background events of negative weight enter with the opposite sign, zero drops out
     w = [torch.tensor(np.where(np.arange(n) % 7 == 3, 0.0, rng.uniform(0.5 if k == 0 else -0.4, 1.5, n)), device=dev)
          if use else None for k, (n, use) in enumerate(zip(sizes, weights))]
+    if len(few):
+        w[1][::5][:len(few)] = torch.tensor(few, dtype=torch.float64, device=dev)
     ana = ctpwa_b200.analysis.from_device(str(cfg), s[0], s[1], s[2], weights=w)
     p = torch.tensor(workloads.true_params(ana.getNVector(), ana.getFreeResParams()[0].numpy(), seed=seed) *
                      rng.uniform(0.97, 1.03, ana.getNParams()), device=dev)
+    return ana, p
+
+
+def _check(ana, p):
+    import torch
+
     H = ana.getHessian(p)
-    F = ana.getHessianVectorProduct(p, torch.eye(p.numel(), dtype=torch.float64, device=dev))
+    F = ana.getHessianVectorProduct(p, torch.eye(p.numel(), dtype=torch.float64, device=p.device))
     F = 0.5 * (F + F.T)
     assert torch.isfinite(F).all() and float(F.abs().max()) > 0
     assert float((H - F).abs().max()) <= 1e-11 * float(F.abs().max())
     assert torch.equal(H, ana.getHessian(p))  # fixed summation order
+
+
+def _compare(tmp_path, text, masses, sizes, weights=(False, False, False), seed=1):
+    _check(*_setup(tmp_path, text, masses, sizes, weights, seed))
 
 
 @pytest.mark.parametrize("sizes", [(1, 1, 0), (31, 33, 1), (32, 32, 32), (129, 127, 63), (40_000, 4_001, 395)])
@@ -97,3 +110,46 @@ def test_capture_of_the_first_call(tmp_path):
     g.replay()
     torch.cuda.synchronize()
     assert torch.equal(H, ana.getHessian(p))
+
+
+# Clamped events: components of w S / f beyond 1e10 count as constants. Weights
+# of 1e12 clamp some of an event's components, 1e18 all of them.
+CLAMPING = {"some": [1e12, -1e12, 3e12, 1e10, -2e11, 1e12], "all": [1e18, -1e18, 1e18, 1.0, 1e18]}
+
+
+@pytest.mark.parametrize("few", list(CLAMPING))
+@pytest.mark.parametrize("model", ["pipi_3rho", "ksks", "kkpi"])
+@pytest.mark.parametrize("paired", [True, False])
+def test_clamped_by_weight(tmp_path, monkeypatch, model, paired, few):
+    from ctpwa_b200 import workloads
+
+    if not paired:
+        monkeypatch.setenv("CTPWA_NO_POL_PAIRING", "1")
+    _check(*_setup(tmp_path, workloads.config_text(model, "p", "d"), workloads.MASSES[model], (1001, 217, 40),
+                   weights=(False, True, False), seed=7, few=CLAMPING[few]))
+
+
+@pytest.mark.parametrize("paired", [True, False])
+def test_clamped_at_an_amplitude_zero(tmp_path, monkeypatch, paired):
+    """One coupling set so that the amplitude of one data event vanishes to rounding: its S / f lies beyond 1e10 at
+    unit weight, and what it would add to the Hessian unclamped is 1e20 times what the other events add."""
+    import torch
+
+    from ctpwa_b200 import workloads
+
+    if not paired:
+        monkeypatch.setenv("CTPWA_NO_POL_PAIRING", "1")
+    ana, p = _setup(tmp_path, workloads.config_text("kkpi", "p", "d"), workloads.MASSES["kkpi"], (1001, 217, 40), seed=9)
+    nV = ana.getNVector()
+
+    def f(z):  # all amplitudes of one event share one angular vector: f = |A + z B|^2
+        q = p.clone()
+        q[1], q[nV + 1] = z.real, z.imag
+        return float(ana.getIntensity(q, kind=1)[3])
+
+    a, k, b = f(0j), f(1 + 0j), f(1j)
+    bb = (f(1 + 0j) + f(-1 + 0j) - 2 * a) / 2  # |B|^2
+    z = -complex(k - a - bb, b - a - bb) / (2 * bb)
+    p[1], p[nV + 1] = z.real, z.imag
+    assert f(z) < 1e-20 * a
+    _check(ana, p)
