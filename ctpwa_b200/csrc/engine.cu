@@ -1094,6 +1094,7 @@ Engine::~Engine()
     devFree(d_hvsums_);
     devFree(d_htsums_);
     devFree(d_hess_img_);
+    devFree(d_hess_clamped_);
     devFree(d_hess_rows_);
     devFree(d_hess_sums_);
     devFree(d_gpart_);
@@ -2898,6 +2899,7 @@ struct CtHvpArgsH {
     double* rows;
     int ctas;
     int pad;
+    const int* gate;
 };
 
 // argument blocks of the one-pass Hessian kernels (must match kernels/hessgram.cuh)
@@ -2920,6 +2922,7 @@ struct CtHessArgsH {
     const double* v;
     void* img;
     double* rows;
+    int* clamped;
 };
 struct CtHessGroupsH {
     int beg[4], cnt[4];
@@ -2957,8 +2960,9 @@ namespace {
 // one warp per (sample, column), fixed order.
 __global__ void __launch_bounds__(1024) ct_hvp_rowsum_kernel(const double* __restrict__ rows, int ctas, int nacc,
                                                              int c0, int n0, int c1, int n1, int c2, int n2,
-                                                             double* __restrict__ out)
+                                                             const int* gate, double* __restrict__ out)
 {
+    if (gate && *gate == 0) return;
     const int d = blockIdx.x;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nwarp = blockDim.x >> 5;
     const int beg[3] = {c0, c1, c2}, cnt[3] = {n0, n1, n2};
@@ -3144,6 +3148,7 @@ void Engine::compileHess()
     }
     hess_grid_ = std::max(1, begin);
     alloc(d_hess_img_, hess_sym_bytes_);
+    alloc(d_hess_clamped_, sizeof(int));
     alloc(d_hess_rows_, sizeof(double) * (size_t)hess_grid_ * h.row);
     alloc(d_hess_sums_, sizeof(double) * 4 * (size_t)h.row);
     k_hess_pro_ = (void*)kp;
@@ -3191,6 +3196,7 @@ void Engine::hessSums(const double* d_params, const double* d_dirs, int ndir, do
     a.v = d_v_;
     a.img = d_hess_img_;
     a.rows = d_hess_rows_;
+    a.clamped = d_hess_clamped_;
     void* args[] = {&a};
     CT_CUDA(cudaLaunchKernel(k_hess_pro_, dim3(1), dim3(512), args, 0, stream));
     CT_CUDA(cudaMemcpyAsync(hess_sym_, d_hess_img_, hess_sym_bytes_, cudaMemcpyDeviceToDevice, stream));
@@ -3231,10 +3237,15 @@ void Engine::hvpSums(const double* d_params, const double* d_dirs, int ndir, dou
                                                             nullptr);
     CT_CUDA(cudaGetLastError());
     hessSums(d_params, d_dirs, ndir, d_tsums, nullptr, stream);
+    // events with clamped components make the second derivatives unsymmetric:
+    // the one pass gives the symmetric part, the sums of a direction are
+    // forward mode's (three launches that return at once without such events)
+    forwardHvpSums(d_params, d_dirs, ndir, d_tsums, stream, d_hess_clamped_);
 }
 
+// gate: device flag; where it is 0 the launches return at once and d_tsums stays as it is
 void Engine::forwardHvpSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums,
-                            cudaStream_t stream)
+                            cudaStream_t stream, const int* gate)
 {
     if (ndir <= 0) return;
     compileHvp();
@@ -3269,6 +3280,7 @@ void Engine::forwardHvpSums(const double* d_params, const double* d_dirs, int nd
     a.consts = d_hconsts_;
     a.rows = d_hrows_;
     a.ctas = hlay_.grid;
+    a.gate = gate;
     for (int d0 = 0; d0 < ndir; d0 += hvp_cap_) {
         const int nd = std::min(hvp_cap_, ndir - d0);
         a.ndir = nd;
@@ -3278,7 +3290,7 @@ void Engine::forwardHvpSums(const double* d_params, const double* d_dirs, int nd
         CT_CUDA(cudaLaunchKernel(k_hvp_, dim3(hlay_.grid, nd), dim3(hvp_block_), args, (size_t)hvp_dsmem_, stream));
         ct_hvp_rowsum_kernel<<<nd, 1024, 0, stream>>>(d_hrows_, hlay_.grid, nacc, hlay_.cta[0][0], hlay_.cta[0][1],
                                                       hlay_.cta[1][0], hlay_.cta[1][1], hlay_.cta[2][0], hlay_.cta[2][1],
-                                                      d_tsums + (size_t)d0 * 3 * nacc);
+                                                      gate, d_tsums + (size_t)d0 * 3 * nacc);
         CT_CUDA(cudaGetLastError());
     }
 }
@@ -3562,7 +3574,7 @@ void Engine::hessianGram(const double* d_params, double* d_hess, cudaStream_t st
         CT_CUDA(cudaMallocAsync((void**)&d_dirs, sizeof(double) * dirs.size(), stream));
         CT_CUDA(cudaMallocAsync((void**)&d_rows, sizeof(double) * dirs.size(), stream));
         CT_CUDA(cudaMemcpyAsync(d_dirs, dirs.data(), sizeof(double) * dirs.size(), cudaMemcpyHostToDevice, stream));
-        hessianRows(d_params, d_dirs, nT, d_rows, stream);
+        hessianRows(d_params, d_dirs, nT, d_rows, stream, false);
         std::vector<double> rows(dirs.size());
         CT_CUDA(cudaMemcpyAsync(rows.data(), d_rows, sizeof(double) * rows.size(), cudaMemcpyDeviceToHost, stream));
         CT_CUDA(cudaFreeAsync(d_dirs, stream));
@@ -3852,8 +3864,11 @@ void Engine::hessianVectorProducts(const double* d_params, const double* d_dirs,
     }
 }
 
-// Rows H u of up to hvp_cap_ directions, by whichever form is faster.
-void Engine::hessianRows(const double* d_params, const double* d_dirs, int ndir, double* d_out, cudaStream_t stream)
+// Rows H u of up to hvp_cap_ directions, by whichever form is faster; with
+// `symmetric` those of the symmetrised matrix where events with clamped
+// components make it unsymmetric, if that is faster.
+void Engine::hessianRows(const double* d_params, const double* d_dirs, int ndir, double* d_out, cudaStream_t stream,
+                         bool symmetric)
 {
     if (!onePassHessian(ndir)) {
         hessianVectorProducts(d_params, d_dirs, ndir, d_out, stream);
@@ -3864,6 +3879,7 @@ void Engine::hessianRows(const double* d_params, const double* d_dirs, int ndir,
                                                             d_err_);
     CT_CUDA(cudaGetLastError());
     hessSums(d_params, d_dirs, ndir, d_htsums_, d_hvsums_, stream);
+    if (!symmetric) forwardHvpSums(d_params, d_dirs, ndir, d_htsums_, stream, d_hess_clamped_);
     finalizeHvp(d_params, d_dirs, ndir, d_hvsums_, d_htsums_, d_out, stream);
 }
 
@@ -3871,7 +3887,7 @@ void Engine::hessianExact(const double* d_params, double* d_hess, cudaStream_t s
 {
     hvpBuffers();
     const int n = model_.nParams();
-    hessianRows(d_params, d_hdirs_, n, d_hess, stream);
+    hessianRows(d_params, d_hdirs_, n, d_hess, stream, true);
     ct_symmetrize_kernel<<<std::max(1, (n * n + 255) / 256), 256, 0, stream>>>(d_hess, n);
     CT_CUDA(cudaGetLastError());
 }

@@ -240,11 +240,13 @@ private:
     void compileKernel();
     void compileHvp();
     void hvpBuffers();
-    void forwardHvpSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums, cudaStream_t stream);
+    void forwardHvpSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums, cudaStream_t stream,
+                        const int* gate = nullptr);
     // one-pass Hessian sums (kernels/hessgram.cuh; compiled and allocated on first use)
     void compileHess();
     bool onePassHessian(int ndir) const;
-    void hessianRows(const double* d_params, const double* d_dirs, int ndir, double* d_out, cudaStream_t stream);
+    void hessianRows(const double* d_params, const double* d_dirs, int ndir, double* d_out, cudaStream_t stream,
+                     bool symmetric);
     void hessSums(const double* d_params, const double* d_dirs, int ndir, double* d_tsums, double* d_vsums,
                   cudaStream_t stream);
     void* k_hess_pro_ = nullptr;
@@ -254,6 +256,7 @@ private:
     void* hess_sym_ = nullptr;  // the module's constant block and its image
     size_t hess_sym_bytes_ = 0;
     void* d_hess_img_ = nullptr;
+    int* d_hess_clamped_ = nullptr;  // set by a pass that met events with clamped components
     int hess_lay_[4][2] = {};   // first CTA and CTAs of phase space, data, background, weighted phase space
     int hess_grid_ = 0;
     double* d_hess_rows_ = nullptr;

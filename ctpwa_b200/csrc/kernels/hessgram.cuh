@@ -37,7 +37,9 @@
 //
 // Clamps as in the gradient pass: components of w S / f beyond 1e10 count as
 // constants (no derivative). Only then are the weights of a polarisation's
-// columns masks, and the rank-one term becomes that of two different vectors.
+// columns masks, and the rank-one term becomes that of two different vectors,
+// of which the symmetric part is kept: what a symmetrised Hessian needs. For
+// single rows the caller runs forward mode where `clamped` is set.
 //
 // Each warp strides over 32-event tiles of its CTA's sample; each CTA writes
 // one row [HT][8][8] blocks, [M_HLIN] linear sums, sum -w log f; fixed orders
@@ -98,6 +100,7 @@ struct CtHessArgs {
     const double* v;    // couplings (re, im) x M_NA
     CtHessConsts* img;  // image of hs_k, written by ct_hess_prologue
     double* rows;       // [CTAs][CT_HROW]
+    int* clamped;       // set to 1 when an event had clamped components
 };
 
 // parameter-only constants (one warp per part, up to 16) and couplings
@@ -106,6 +109,7 @@ extern "C" __global__ void __launch_bounds__(512) ct_hess_prologue(CtHessArgs A)
     if ((threadIdx.x & 31) == 0)
         for (int q = threadIdx.x >> 5; q < M_NHPRO; q += 16) hs_prologue(q, A.theta, A.img->c);
     for (int i = threadIdx.x; i < 2 * M_NA; i += 512) A.img->v[i] = A.v[i];
+    if (threadIdx.x == 0) *A.clamped = 0;
 }
 
 __device__ __forceinline__ void ct_dmma(double (&c)[2], double a, double b)
@@ -500,6 +504,7 @@ extern "C" __global__ void __launch_bounds__(32 * CT_HESS_WARPS, CT_HESS_MINB) c
         if (!T.active) T.we = 0.0;
         hs_columns(ev, hs_k.c, T);
         T.finish();
+        if (T.any && lane == 0) *A.clamped = 1;
     }
     // CTA sums: every warp's sums to its part of shared memory, then added in warp order
     __syncthreads();

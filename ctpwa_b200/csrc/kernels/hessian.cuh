@@ -140,6 +140,7 @@ struct CtHvpArgs {
     double* rows;         // [ndir][ctas][CT_HNACC] tangent sums
     int ctas;             // CTAs per direction
     int pad;
+    const int* gate;      // nothing is done where it points to 0 (nullptr: always done)
 };
 
 // One thread per direction: the parameter-only subexpressions and their
@@ -147,7 +148,7 @@ struct CtHvpArgs {
 extern "C" __global__ void ct_hvp_prologue(CtHvpArgs A)
 {
     const int d = blockIdx.x;
-    if (threadIdx.x != 0 || d >= A.ndir) return;
+    if (threadIdx.x != 0 || d >= A.ndir || (A.gate && *A.gate == 0)) return;
     CtDual th[M_NTH > 0 ? M_NTH : 1];
     const double* u = A.dirs + (long long)d * A.nparam + 2 * A.nc;
 #pragma unroll 1
@@ -169,6 +170,7 @@ __device__ __forceinline__ CtDual ct_clamp(CtDual x, double k)
 
 extern "C" __global__ void __launch_bounds__(CT_HVP_BLOCK) ct_hvp_f64(CtHvpArgs A)
 {
+    if (A.gate && *A.gate == 0) return;
     const int d = blockIdx.y, cta = blockIdx.x;
     int si = 0;
 #pragma unroll

@@ -153,3 +153,24 @@ def test_clamped_at_an_amplitude_zero(tmp_path, monkeypatch, paired):
     p[1], p[nV + 1] = z.real, z.imag
     assert f(z) < 1e-20 * a
     _check(ana, p)
+
+
+def test_clamped_products_are_rows(tmp_path):
+    """With clamped events the matrix of second derivatives is not symmetric. Only getHessian symmetrises it: the
+    sums of a shard along several directions are those of each direction alone, and the resonance rows of the
+    Gram-based Hessian are the products."""
+    import torch
+
+    from ctpwa_b200 import workloads
+
+    ana, p = _setup(tmp_path, workloads.config_text("kkpi", "p", "d"), workloads.MASSES["kkpi"], (1001, 217, 40),
+                    weights=(False, True, False), seed=7, few=CLAMPING["some"])
+    n, nV = p.numel(), ana.getNVector()
+    d = torch.tensor(np.random.default_rng(3).standard_normal((6, n)), device=p.device)
+    for dirs in (d, torch.eye(n, dtype=torch.float64, device=p.device)):
+        many = ana.getShardHvpSums(p, dirs).view(dirs.shape[0], -1)
+        one = torch.stack([ana.getShardHvpSums(p, u[None]).view(-1) for u in dirs])
+        assert float((many - one).abs().max()) <= 1e-11 * float(one.abs().max())
+    rows = ana.getHessianVectorProduct(p, torch.eye(n, dtype=torch.float64, device=p.device))[2 * nV:]
+    G = ana.getHessian(p, method="gram")[2 * nV:]
+    assert float((rows[:, :2 * nV] - G[:, :2 * nV]).abs().max()) <= 1e-11 * float(rows.abs().max())
