@@ -2123,7 +2123,7 @@ HessShape hessShape(const GeneratedModel& gen)
 {
     HessShape h;
     const int hp = gen.ngrad, hb = (hp + 7) / 8;
-    if (gen.hess_header.empty() || hp < 1 || hb > 6) return h;
+    if (gen.hess_header.empty() || hp < 1 || hb > 6 || gen.npol > 16) return h;
     h.blocks = hb;
     h.row = hb * (hb + 1) / 2 * 64 + gen.nhlin + 1;
     const int slab = std::max(std::max(8 * hb * 68, 32 * 33) + 68, h.row);  // CT_HSLAB, reused for the CTA's row

@@ -131,6 +131,7 @@ struct CtHessTile {
     double cr[M_NPLANE], ci[M_NPLANE];  // sum_p SL_{c,p} conj(u_p), u the clamped w S / f
     double we, alpha, nlog;
     unsigned mask;  // clamped components, 2 p + (0 re, 1 im)
+    static_assert(M_NPOL <= 16, "mask of clamped components");
     bool any;       // some lane of the warp clamps
     int kind;
     bool active;

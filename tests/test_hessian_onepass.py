@@ -174,3 +174,32 @@ def test_clamped_products_are_rows(tmp_path):
     rows = ana.getHessianVectorProduct(p, torch.eye(n, dtype=torch.float64, device=p.device))[2 * nV:]
     G = ana.getHessian(p, method="gram")[2 * nV:]
     assert float((rows[:, :2 * nV] - G[:, :2 * nV]).abs().max()) <= 1e-11 * float(rows.abs().max())
+
+
+def test_many_polarisations(tmp_path):
+    """27 polarisation states (a vector decaying to two vectors and a pseudoscalar), whose components a 32-bit mask
+    does not hold: forward mode."""
+    text = """Particles:
+  Jpsi: {J: 1, P: -1, mass: 3.0969}
+  V1:   {J: 1, P: -1, mass: 0.78265}
+  V2:   {J: 1, P: -1, mass: 0.77526}
+  pi0:  {J: 0, P: -1, mass: 0.13495}
+Data:
+  order: [V1, V2, pi0]
+  data: [npy, "d"]
+  phsp: [npy, "p"]
+DecayChains:
+  c:
+    Jpsi: [[pi0, R]]
+    R: [V1, V2]
+    intermediates:
+      R:
+        - [J: 0, P: -1]: [eta1760, eta2225]
+Resonances:
+  eta1760: {J: 0, P: -1, model: BWR, parameters: [1.76, 0.24], free: [0, 1]}
+  eta2225: {J: 0, P: -1, model: BWR, parameters: [2.22, 0.18], free: [0, 1]}
+"""
+    ana, p = _setup(tmp_path, text, (0.78265, 0.77526, 0.13495), (301, 97, 0), weights=(False, True, False), seed=7,
+                    few=CLAMPING["some"])
+    assert ana.getNPolarizations() == 27
+    _check(ana, p)
