@@ -18,8 +18,10 @@
 
 #include "angular.cuh"
 
+#include <dirent.h>
 #include <dlfcn.h>
 #include <nvrtc.h>
+#include <sys/stat.h>
 #include <unistd.h>
 
 #include <algorithm>
@@ -806,9 +808,10 @@ std::string cacheDir()
 // (the per-call constant block is a module global, and handles on different
 // streams must not share it), but loading one costs 1-1.5 ms, most of a small
 // toy job's set-up: a handle that goes returns its modules here, and the next
-// handle of the same generated code, options and device takes them over
-// (its first call rewrites the constant block). At most kMax modules wait;
-// beyond that the one idle longest is unloaded.
+// handle of the same generated code, kernel sources, options and device takes
+// them over. Its first call rewrites the constant block, so a module comes
+// here only when no kernel of it runs any more (~Engine waits). At most kMax
+// modules wait; beyond that the one idle longest is unloaded.
 class ModulePool {
 public:
     static constexpr size_t kMax = 16;
@@ -1054,8 +1057,23 @@ Engine::Engine(const std::string& config_path, const EngineOptions& opt) : opt_(
     init_stream_ = nullptr;
 }
 
+// Waits for all work on the handle's device: kernels that the caller has
+// queued on streams of its own still read the handle's memory and modules,
+// which the next handle takes over. False when it could not (a stream of the
+// device is being captured, or an earlier error).
+bool Engine::waitForDevice() const
+{
+    int cur = 0;
+    if (cudaGetDevice(&cur) != cudaSuccess || cudaSetDevice(opt_.device) != cudaSuccess) return false;
+    const bool ok = cudaDeviceSynchronize() == cudaSuccess;
+    if (!ok) cudaGetLastError();
+    cudaSetDevice(cur);
+    return ok;
+}
+
 Engine::~Engine()
 {
+    const bool idle = waitForDevice();
     for (auto& s : samples_) {
         devFree(s.p4);
         devFree(s.slamp64);
@@ -1106,7 +1124,10 @@ Engine::~Engine()
         cudaStreamSynchronize(mem_stream_);
         cudaStreamDestroy(mem_stream_);
     }
-    for (auto& m : modules_) ModulePool::get().give(m.first, (cudaLibrary_t)m.second);
+    for (auto& m : modules_) {
+        if (idle) ModulePool::get().give(m.first, (cudaLibrary_t)m.second);
+        else cudaLibraryUnload((cudaLibrary_t)m.second);
+    }
 }
 
 void Engine::loadSamples()
@@ -2114,8 +2135,10 @@ std::string jitHvpCubin(const GeneratedModel& gen, bool paired, bool* cache_hit)
 // Launch of the one-pass Hessian kernel (kernels/hessgram.cuh): blocks of 8
 // rows of the matrix, warps per CTA, minimum resident CTAs per SM, doubles of
 // one CTA row and dynamic shared memory. blocks == 0: the model has no
-// one-pass form, or its matrix has more than 48 rows (21 blocks of
-// accumulators, 84 registers a thread).
+// one-pass form, its matrix has more than 48 rows (21 blocks of accumulators,
+// 84 registers a thread; three chains of rho with 48 rows, 1.1M events: 1.93 ms
+// against 16.8 ms in forward mode), or it has more than 16 polarisation states
+// (the kernel's mask of clamped components is one 32-bit word).
 struct HessShape {
     int blocks = 0, warps = 4, minb = 2, row = 0, dsmem = 0;
 };
@@ -2194,6 +2217,25 @@ bool angularInterpreted()
     return e && *e && *e != '0';
 }
 
+// The kernel sources that a module compiled now is made of: their folder and
+// the sizes and times of its files (10 us; reading and hashing them would be
+// a good part of what the pool saves).
+std::string kernelStamp()
+{
+    const std::string dir = kernelDir();
+    uint64_t sum = 0;
+    if (DIR* d = opendir(dir.c_str())) {
+        while (const dirent* e = readdir(d)) {
+            struct stat st;
+            if (e->d_name[0] == '.' || fstatat(dirfd(d), e->d_name, &st, 0) != 0) continue;
+            sum += fnv1a(std::string(e->d_name) + " " + std::to_string(st.st_size) + " " + std::to_string(st.st_mtim.tv_sec) +
+                         " " + std::to_string(st.st_mtim.tv_nsec));
+        }
+        closedir(d);
+    }
+    return dir + " " + std::to_string(sum);
+}
+
 std::string shapeKey(const FusedShape& sh)
 {
     std::string k;
@@ -2207,7 +2249,7 @@ std::string shapeKey(const FusedShape& sh)
 template <class Cubin>
 void* Engine::takeModule(const std::string& kind, const Cubin& cubin)
 {
-    const std::string key = gen_.id + " " + std::to_string(opt_.device) + " " + kind;
+    const std::string key = gen_.id + " " + std::to_string(opt_.device) + " " + kind + " " + kernelStamp();
     cudaLibrary_t lib = ModulePool::get().take(key);
     if (!lib) {
         const std::string image = cubin();
@@ -2223,6 +2265,7 @@ void Engine::compileKernel()
 {
     auto t0 = std::chrono::steady_clock::now();
     cudaLibrary_t lib = (cudaLibrary_t)takeModule("fused " + shapeKey(shape_), [&] { return jitCubin(gen_, &jit_cache_hit_); });
+    image_key_ = (const void*)(uintptr_t)fnv1a(modules_.back().first);
     cudaKernel_t k64, kmx, kin, kpro;
     CT_CUDA(cudaLibraryGetKernel(&kpro, lib, "ct_prologue"));
     k_pro_ = (void*)kpro;
@@ -2266,13 +2309,6 @@ void Engine::compileKernel()
                 CT_CUDA(cudaFuncSetAttribute((const void*)k, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              std::max(shape_.dsmem[pr], pr == 0 ? shape_.dsmem_pc : 0)));
     k_int_ = (void*)kin;
-    {
-        std::string key = gen_.id;
-        for (int pr = 0; pr < 2; ++pr)
-            key += "|" + std::to_string(shape_.block[pr]) + "," + std::to_string(shape_.minb[pr]) + "," +
-                   std::to_string(shape_.dsmem[pr]);
-        image_key_ = (const void*)(uintptr_t)fnv1a(key);
-    }
     jit_seconds_ = std::chrono::duration<double>(std::chrono::steady_clock::now() - t0).count();
 }
 

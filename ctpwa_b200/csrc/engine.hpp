@@ -281,6 +281,7 @@ private:
     std::vector<std::pair<std::string, void*>> modules_;
     template <class Cubin>
     void* takeModule(const std::string& kind, const Cubin& cubin);
+    bool waitForDevice() const;
     void* k_f64_ = nullptr;
     void* k_mixed_ = nullptr;
     void* k_int_ = nullptr;
