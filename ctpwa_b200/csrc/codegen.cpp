@@ -1140,7 +1140,9 @@ std::string Gen::emit()
     std::vector<int> adjConst;              // nodes of the summed adjoints
     bool reverse = true;
     {
-        // nodes reached from the outputs without going into a branch
+        // nodes reached from the outputs without going into a branch (nor
+        // through a condition, which passes no adjoint: a guarded r in
+        // r == 0 ? c : r is both, and where it is replaced its adjoint is zero)
         std::vector<char> plain(N.size(), 0);
         std::vector<int> st;
         for (const auto& c : cols)
@@ -1150,10 +1152,7 @@ std::string Gen::emit()
             st.pop_back();
             if (x < 0 || plain[x]) continue;
             plain[x] = 1;
-            if (N[x].op == dag::Sel) {
-                st.push_back(N[x].c);
-                continue;
-            }
+            if (N[x].op == dag::Sel) continue;
             for (int k : {N[x].a, N[x].b, N[x].c}) st.push_back(k);
         }
         for (size_t x = 0; x < N.size(); ++x) {
