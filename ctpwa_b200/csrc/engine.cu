@@ -1753,6 +1753,7 @@ void Engine::pairPolarisations()
     for (int pr = 0; pr < 2; ++pr)
         if (paired_[pr]) (pr == 0 ? k_f64_ : k_mixed_) = k_pc_[pr];
     if (paired_[0]) {
+        shape_.block[0] = shape_.block_pc;
         shape_.stage[0] = shape_.stage_pc;
         shape_.dsmem[0] = shape_.dsmem_pc;
     }
@@ -1933,21 +1934,11 @@ FusedShape fusedShape(const GeneratedModel& gen)
         if (v < lo || v > hi) throw std::runtime_error(std::string(name) + " out of range");
         return v;
     };
-    // plain path: 256 threads where the sums and the copies of paired
-    // polarisations fit twice per SM (16 warps, at 128 registers), else 192
-    // (12 warps): three chains of rho 5.55M events 0.262 ms against 0.287 ms,
-    // K_S K_S 1.1M events 0.045 against 0.047 ms; K+K-pi0 has room for 192
-    // only (256 with direct loads 0.61 ms against 0.56 ms)
-    const long long f64_bytes = (gen.nsum[0] + (long long)std::max(1, gen.nplane) * std::max(1, gen.npol) + gen.nev64) * 8;
-    sh.block[0] = get("CTPWA_F64_BLOCK", 2 * (f64_bytes * 256 + 8 * 1024) <= 228 * 1024 ? 256 : 192, 32, 1024);
+    sh.acc[0] = get("CTPWA_F64_ACC_SMEM", 1, 0, 1);
+    sh.acc[1] = get("CTPWA_MX_ACC_SMEM", 0, 0, 1);
     sh.minb[0] = get("CTPWA_F64_MINB", 2, 1, 16);
     sh.block[1] = get("CTPWA_MX_BLOCK", 256, 32, 1024);
     sh.minb[1] = get("CTPWA_MX_MINB", 2, 1, 16);
-    sh.acc[0] = get("CTPWA_F64_ACC_SMEM", 1, 0, 1);
-    sh.acc[1] = get("CTPWA_MX_ACC_SMEM", 0, 0, 1);
-
-    for (int i = 0; i < 2; ++i)
-        if (sh.block[i] % 32) throw std::runtime_error("fused block sizes must be multiples of 32");
     // Staging of the event tables through shared memory, used when its
     // buffers fit at the requested residency next to the static shared
     // memory: 1 the frontier rows and 2 the frontier and angular rows, by
@@ -1966,31 +1957,46 @@ FusedShape fusedShape(const GeneratedModel& gen)
     auto fits = [&](int i, long long bytes) {
         return bytes + reserve <= per_cta && (long long)sh.minb[i] * (bytes + reserve) <= per_sm;
     };
-    for (int i = 0; i < 2; ++i) {
-        // dynamic shared memory = [gradient-sum slots][two tile buffers]
-        long long acc_bytes = sh.acc[i] ? (gen.nsum[i] * sh.block[i] * accb[i] + 127) / 128 * 128 : 0;
-        if (!fits(i, acc_bytes)) {
-            sh.acc[i] = 0;
-            acc_bytes = 0;
-        }
-        long long npl = (long long)std::max(1, gen.nplane) * std::max(1, gen.npol);
-        if (i == 1) npl = (npl + 1) / 2 * 2;  // FP32 angular records of an even number of values
+    // dynamic shared memory = [gradient-sum slots][tile buffers]
+    const long long pairs = (long long)std::max(1, gen.nplane) * std::max(1, gen.npol);
+    auto sums = [&](int i, int block) { return (gen.nsum[i] * block * accb[i] + 127) / 128 * 128; };
+    // bytes of one event's FP64 values in mode 4, complex or paired angular values
+    const long long staged[2] = {pairs * rowb[0] + 8LL * gen.nev64, (pairs + gen.nev64) * 8LL};
+    // Plain path, for either table: 256 threads where the sums and the copies
+    // of mode 4 fit twice per SM (16 warps, at 128 registers), else 192 (12
+    // warps). Paired: three chains of rho 5.55M events 0.262 ms against
+    // 0.287 ms, K_S K_S 1.1M events 0.045 against 0.047 ms; K+K-pi0 has room
+    // for 192 only (256 with direct loads 0.61 ms against 0.56 ms). Unpaired
+    // (whole evaluations): three chains of rho have room for 192, 0.353 ms
+    // against 0.399 ms with direct loads at 256; one chain 41 us at 256 and 42
+    // at 192, K_S K_S 77 and 74 us.
+    auto f64_block = [&](int paired) {
+        return fits(0, sums(0, 256) + staged[paired] * 256) ? 256 : 192;
+    };
+    sh.block[0] = get("CTPWA_F64_BLOCK", f64_block(0), 32, 1024);
+    sh.block_pc = get("CTPWA_F64_BLOCK", f64_block(1), 32, 1024);
+    sh.block[1] = get("CTPWA_MX_BLOCK", 256, 32, 1024);
+    for (int b : {sh.block[0], sh.block[1], sh.block_pc})
+        if (b % 32) throw std::runtime_error("fused block sizes must be multiples of 32");
+    sh.acc[0] = sh.acc[0] && fits(0, sums(0, std::max(sh.block[0], sh.block_pc)));
+    sh.acc[1] = sh.acc[1] && fits(1, sums(1, sh.block[1]));
+    // v 0, 1: the plain and the mixed kernel; 2: the plain one for paired polarisations
+    for (int v = 0; v < 3; ++v) {
+        const int i = v == 1, block = v == 2 ? sh.block_pc : sh.block[v];
+        const long long acc_bytes = sh.acc[i] ? sums(i, block) : 0;
+        const long long npl = i == 1 ? (pairs + 1) / 2 * 2 : pairs;  // FP32 angular records of an even number of values
         const long long evb = i == 0 ? 8LL * gen.nev64 : 4LL * evfStride(gen) + 8LL * gen.nevd;  // frontier bytes per event
         const int stage_on = stage_req[i];
-        long long stage_bytes = 2LL * ((stage_on == 2 ? npl * rowb[i] : 0) + evb) * sh.block[i];
+        long long stage_bytes = 2LL * ((stage_on == 2 ? npl * rowb[i] : 0) + evb) * block;
         if (stage_on == 3) {
             // [2][NA][block] values of the table's type (16-byte rounded), then [2][NB][block] FP64
             const long long na = i == 0 ? gen.nev64 : evfStride(gen), nb = i == 0 ? 0 : gen.nevd, sz = i == 0 ? 8 : 4;
-            stage_bytes = (2LL * std::max(1LL, na) * sh.block[i] * sz + 15) / 16 * 16 + 2LL * nb * sh.block[i] * 8;
+            stage_bytes = (2LL * std::max(1LL, na) * block * sz + 15) / 16 * 16 + 2LL * nb * block * 8;
         }
-        if (stage_on == 4) stage_bytes = (npl * rowb[0] + 8LL * gen.nev64) * sh.block[0];
-        if (stage_on && fits(i, acc_bytes + stage_bytes)) sh.stage[i] = stage_on;
-        sh.dsmem[i] = (int)(acc_bytes + (sh.stage[i] ? stage_bytes : 0));
-        if (i == 0) {
-            if (stage_on == 4) stage_bytes = (npl + gen.nev64) * 8LL * sh.block[0];
-            if (stage_on && fits(0, acc_bytes + stage_bytes)) sh.stage_pc = stage_on;
-            sh.dsmem_pc = (int)(acc_bytes + (sh.stage_pc ? stage_bytes : 0));
-        }
+        if (stage_on == 4) stage_bytes = staged[v == 2] * block;
+        const int on = stage_on && fits(i, acc_bytes + stage_bytes) ? stage_on : 0;
+        (v == 2 ? sh.stage_pc : sh.stage[v]) = on;
+        (v == 2 ? sh.dsmem_pc : sh.dsmem[v]) = (int)(acc_bytes + (on ? stage_bytes : 0));
     }
     return sh;
 }
@@ -2097,6 +2103,7 @@ std::string jitCubin(const GeneratedModel& gen, bool* cache_hit)
     optv.push_back("-DCT_MX_STAGE=" + std::to_string(sh.stage[1]));
 
     optv.push_back("-DCT_F64_BLOCK=" + std::to_string(sh.block[0]));
+    optv.push_back("-DCT_F64_PC_BLOCK=" + std::to_string(sh.block_pc));
     optv.push_back("-DCT_F64_MINB=" + std::to_string(sh.minb[0]));
     optv.push_back("-DCT_MX_BLOCK=" + std::to_string(sh.block[1]));
     optv.push_back("-DCT_MX_MINB=" + std::to_string(sh.minb[1]));
@@ -2240,7 +2247,7 @@ std::string shapeKey(const FusedShape& sh)
 {
     std::string k;
     for (int i = 0; i < 2; ++i)
-        for (int v : {sh.block[i], sh.minb[i], sh.acc[i], sh.stage[i], sh.stage_pc}) k += std::to_string(v) + " ";
+        for (int v : {sh.block[i], sh.minb[i], sh.acc[i], sh.stage[i], sh.block_pc, sh.stage_pc}) k += std::to_string(v) + " ";
     return k;
 }
 

@@ -29,8 +29,9 @@ struct FusedShape {
     int acc[2] = {1, 0};  // per-thread gradient sums in shared memory
     int dsmem[2] = {0, 0};
     // the plain kernel's variant for paired polarisations, whose angular
-    // records are smaller; they become stage[0] and dsmem[0] once the samples
-    // are found to be paired
+    // records are smaller; they become block[0], stage[0] and dsmem[0] once the
+    // samples are found to be paired
+    int block_pc = 192;
     int stage_pc = 0;
     int dsmem_pc = 0;
 };

@@ -881,6 +881,9 @@ __device__ __forceinline__ void ct_fused_body(const CtArgs& A)
 #ifndef CT_F64_BLOCK
 #define CT_F64_BLOCK 192
 #endif
+#ifndef CT_F64_PC_BLOCK  // the variant for paired polarisations
+#define CT_F64_PC_BLOCK CT_F64_BLOCK
+#endif
 #ifndef CT_F64_MINB
 #define CT_F64_MINB 2
 #endif
@@ -894,9 +897,9 @@ extern "C" __global__ void __launch_bounds__(CT_F64_BLOCK, CT_F64_MINB) ct_fused
 {
     ct_fused_body<double, double, false, CT_F64_BLOCK, CT_F64_STAGE, CT_F64_ACC != 0, false>(a);
 }
-extern "C" __global__ void __launch_bounds__(CT_F64_BLOCK, CT_F64_MINB) ct_fused_f64_pc(CtArgs a)
+extern "C" __global__ void __launch_bounds__(CT_F64_PC_BLOCK, CT_F64_MINB) ct_fused_f64_pc(CtArgs a)
 {
-    ct_fused_body<double, double, false, CT_F64_BLOCK, CT_F64_PC_STAGE, CT_F64_ACC != 0, true>(a);
+    ct_fused_body<double, double, false, CT_F64_PC_BLOCK, CT_F64_PC_STAGE, CT_F64_ACC != 0, true>(a);
 }
 // mixed form (FP32 lineshapes and algebra, FP64 logs and sums), all samples
 extern "C" __global__ void __launch_bounds__(CT_MX_BLOCK, CT_MX_MINB) ct_fused_mixed(CtArgs a)
@@ -924,10 +927,10 @@ extern "C" __global__ void __launch_bounds__(CT_F64_BLOCK, CT_F64_MINB)
     ct_fused_body<double, double, false, CT_F64_BLOCK, CT_F64_STAGE, CT_F64_ACC != 0, false, true>(
         jobs[ct_multi_job(cta_off, njobs)]);
 }
-extern "C" __global__ void __launch_bounds__(CT_F64_BLOCK, CT_F64_MINB)
+extern "C" __global__ void __launch_bounds__(CT_F64_PC_BLOCK, CT_F64_MINB)
     ct_fused_f64_pc_multi(const CtArgs* __restrict__ jobs, const int* __restrict__ cta_off, int njobs)
 {
-    ct_fused_body<double, double, false, CT_F64_BLOCK, CT_F64_PC_STAGE, CT_F64_ACC != 0, true, true>(
+    ct_fused_body<double, double, false, CT_F64_PC_BLOCK, CT_F64_PC_STAGE, CT_F64_ACC != 0, true, true>(
         jobs[ct_multi_job(cta_off, njobs)]);
 }
 extern "C" __global__ void __launch_bounds__(CT_MX_BLOCK, CT_MX_MINB)

@@ -69,3 +69,30 @@ def test_two_of_three_polarisations(tmp_path):
     onll, og, _ = Oracle(cfg).nll_grad(p)
     assert abs(float(n) - onll) <= 1e-10 * abs(onll)
     assert np.max(np.abs(g.cpu().numpy() - og)) <= 1e-9 * np.max(np.abs(og))
+
+
+@pytest.mark.parametrize("model", ["pipi_rho", "pipi_3rho", "ksks"])
+@pytest.mark.parametrize("sizes,weighted", [((1, 1, 0), False), ((191, 193, 1), True), ((255, 257, 129), False),
+                                            ((170_003, 17_001, 1_003), True)])
+def test_copies_of_the_complex_table(tmp_path, monkeypatch, model, sizes, weighted):
+    """Samples whose polarisations are not paired: copies of the complex angular values against direct loads."""
+    import torch
+    import ctpwa_b200
+    from ctpwa_b200 import workloads
+
+    cfg, s, w = _setup(tmp_path, model, sizes, weighted)
+    monkeypatch.setenv("CTPWA_NO_POL_PAIRING", "1")
+
+    def evaluate():
+        ana = ctpwa_b200.analysis.from_device(cfg, s[0], s[1], s[2], weights=w)
+        p = torch.tensor(workloads.true_params(ana.getNVector(), ana.getFreeResParams()[0].numpy()) * 1.01, device="cuda:0")
+        n, g = ana.getNLLAndGrad(p)
+        return ana.launchShape()["fp64"], float(n), g
+
+    shape, n1, g1 = evaluate()
+    assert shape["pol_paired"] == 0 and shape["stage"] == 4, shape
+    monkeypatch.setenv("CTPWA_STAGE", "0")
+    direct, n0, g0 = evaluate()
+    assert direct["stage"] == 0 and direct["pol_paired"] == 0
+    assert abs(n1 - n0) <= 1e-12 * max(1.0, abs(n0))
+    assert float((g1 - g0).abs().max()) <= 1e-10 * float(g0.abs().max())
