@@ -1175,6 +1175,17 @@ std::string Gen::emit()
         }
         for (size_t x = 0; x < used.size(); ++x)
             if (used[x]) adjConst.push_back((int)x);
+        // The adjoints are more sums per thread than the thetas. Reverse mode
+        // pays while its sums and the kernel's copies of an event fit in
+        // shared memory: three chains of 7 resonances, 77 sums against 56,
+        // 322 us against 336 us with symbolic derivatives (2.2M events, 128
+        // threads), 8 resonances 361 against 365 us, but 9 resonances (no room
+        // for the copies) 495 against 421 us.
+        const long long values = (long long)out.nplane * m.npol * (m.npol > 1 ? 1 : 2) + out.nev64;
+        if (!smemFits((2LL * m.nAmp() + (long long)adjConst.size() + values) * 8 * kPlainBlockMin, 2)) {
+            reverse = false;
+            adjConst.clear();
+        }
     }
     const int nadj = reverse ? (int)adjConst.size() : m.nTheta();
     std::vector<int> adjOf(N.size(), -1);

@@ -48,6 +48,15 @@ struct GeneratedModel {
     int nevd = 0;
 };
 
+// Whether `bytes` of dynamic shared memory per CTA leave room for `ctas` CTAs
+// per SM (8 KB each for static and reserved shared memory).
+constexpr bool smemFits(long long bytes, int ctas)
+{
+    return bytes + 8 * 1024 <= 227 * 1024 && ctas * (bytes + 8 * 1024) <= 228 * 1024;
+}
+// the smallest block of the plain fused kernel (fusedShape)
+constexpr int kPlainBlockMin = 128;
+
 GeneratedModel generateModel(const Model& m);
 
 // Custom-expression syntax check (throws std::runtime_error like the reference parser).

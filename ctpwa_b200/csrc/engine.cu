@@ -1953,25 +1953,29 @@ FusedShape fusedShape(const GeneratedModel& gen)
     const int stage_req[2] = {st >= 0 ? st : 4, st >= 0 && st < 4 ? st : 3};
     const long long rowb[2] = {16, 8};  // bytes per complex angular value (FP64, FP32)
     const long long accb[2] = {8, 4};   // bytes per gradient sum (FP64, FP32)
-    const long long per_sm = 228LL * 1024, per_cta = 227LL * 1024, reserve = 8LL * 1024;
-    auto fits = [&](int i, long long bytes) {
-        return bytes + reserve <= per_cta && (long long)sh.minb[i] * (bytes + reserve) <= per_sm;
-    };
+    auto fits = [&](int i, long long bytes) { return smemFits(bytes, sh.minb[i]); };
     // dynamic shared memory = [gradient-sum slots][tile buffers]
     const long long pairs = (long long)std::max(1, gen.nplane) * std::max(1, gen.npol);
     auto sums = [&](int i, int block) { return (gen.nsum[i] * block * accb[i] + 127) / 128 * 128; };
     // bytes of one event's FP64 values in mode 4, complex or paired angular values
     const long long staged[2] = {pairs * rowb[0] + 8LL * gen.nev64, (pairs + gen.nev64) * 8LL};
-    // Plain path, for either table: 256 threads where the sums and the copies
-    // of mode 4 fit twice per SM (16 warps, at 128 registers), else 192 (12
-    // warps). Paired: three chains of rho 5.55M events 0.262 ms against
+    // Plain path, for either table: the largest of 256 (128 registers), 192
+    // and 128 threads (255 registers) at which the sums and the copies of mode
+    // 4 fit twice per SM; without room for the copies, 192 or 128 where the
+    // sums fit. Sums in registers spill: three chains of 7 resonances, 77 sums
+    // (2.2M events, whole evaluations), 921 us at 192 against 322 us at 128 in
+    // shared memory; 8 resonances 1224 and 361 us; 6 resonances 335 us at 192
+    // without the copies, 293 us at 128 with them. Paired: three chains of rho 5.55M events 0.262 ms against
     // 0.287 ms, K_S K_S 1.1M events 0.045 against 0.047 ms; K+K-pi0 has room
     // for 192 only (256 with direct loads 0.61 ms against 0.56 ms). Unpaired
     // (whole evaluations): three chains of rho have room for 192, 0.353 ms
     // against 0.399 ms with direct loads at 256; one chain 41 us at 256 and 42
-    // at 192, K_S K_S 77 and 74 us.
+    // at 192, K_S K_S 77 and 74 us; K+K-pi0 5.5M events 0.372 ms at 128 against
+    // 0.449 ms with direct loads at 192.
     auto f64_block = [&](int paired) {
-        return fits(0, sums(0, 256) + staged[paired] * 256) ? 256 : 192;
+        for (int b : {256, 192, kPlainBlockMin})
+            if (fits(0, sums(0, b) + staged[paired] * b)) return b;
+        return !fits(0, sums(0, 192)) && fits(0, sums(0, kPlainBlockMin)) ? kPlainBlockMin : 192;
     };
     sh.block[0] = get("CTPWA_F64_BLOCK", f64_block(0), 32, 1024);
     sh.block_pc = get("CTPWA_F64_BLOCK", f64_block(1), 32, 1024);

@@ -287,7 +287,7 @@ __device__ __forceinline__ void ct_block_reduce_store(const double* accd, const 
                                                       double tscale, const double* __restrict__ J)
 {
     constexpr int N = 2 + ct_nsum<L>;
-    __shared__ double red[BLOCK / 32][N], sum[N];
+    __shared__ double red[BLOCK / 32][N];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
     for (int i = 0; i < N; ++i) {
@@ -301,9 +301,10 @@ __device__ __forceinline__ void ct_block_reduce_store(const double* accd, const 
         double x = 0.0;
 #pragma unroll
         for (int w = 0; w < BLOCK / 32; ++w) x += red[w][i];
-        sum[i] = x;
+        red[0][i] = x;  // (read by this thread only)
     }
     __syncthreads();
+    const double* sum = red[0];
     for (int i = threadIdx.x; i < CT_NACC; i += BLOCK)
         out[i] = i < 2              ? sum[i]
                  : i < 2 + 2 * M_NA ? sum[i] * vscale

@@ -96,3 +96,34 @@ def test_copies_of_the_complex_table(tmp_path, monkeypatch, model, sizes, weight
     assert direct["stage"] == 0 and direct["pol_paired"] == 0
     assert abs(n1 - n0) <= 1e-12 * max(1.0, abs(n0))
     assert float((g1 - g0).abs().max()) <= 1e-10 * float(g0.abs().max())
+
+
+# resonances per chain -> threads, copies; reverse mode up to 8 (88 sums), beyond it symbolic derivatives (72 sums)
+MANY = {5: (128, 4), 7: (128, 4), 8: (128, 4), 9: (128, 4)}
+
+
+@pytest.mark.parametrize("nres", list(MANY))
+def test_many_sums_stay_in_shared_memory(tmp_path, nres):
+    """Three chains of several resonances: the per-thread gradient sums and the copies of an event fit twice per SM at
+    128 threads; against the oracle's FP64 result."""
+    import torch
+    import ctpwa_b200
+    from ctpwa_b200 import workloads
+    from oracle.binding import Oracle
+
+    cfg = workloads.make("pipi_3rho", tmp_path, n_phsp=2003, n_data=301, n_bkg=0, accept_reject=False, seed=3,
+                         gpu_generator=False)
+    names = [f"r{i}" for i in range(nres)]
+    text = open(cfg).read()
+    text = text[:text.index("Resonances:")].replace("rho770, rho1450, rho1700", ", ".join(names)) + "Resonances:\n"
+    for i, n in enumerate(names):
+        text += f"  {n}: {{J: 1, P: -1, model: BWR, parameters: [{0.8 + 0.13 * i:.3f}, {0.15 + 0.02 * i:.3f}], free: [0, 1]}}\n"
+    open(cfg, "w").write(text)
+    ana = ctpwa_b200.analysis(cfg)
+    shape = ana.launchShape()["fp64"]
+    assert shape["acc_smem"] == 1 and (shape["block"], shape["stage"]) == MANY[nres], shape
+    p = workloads.true_params(ana.getNVector(), ana.getFreeResParams()[0].numpy())
+    n, g = ana.getNLLAndGrad(torch.tensor(p, device="cuda:0"))
+    onll, og, _ = Oracle(cfg).nll_grad(p)
+    assert abs(float(n) - onll) <= 1e-10 * abs(onll)
+    assert np.max(np.abs(g.cpu().numpy() - og)) <= 1e-9 * np.max(np.abs(og))
