@@ -3205,9 +3205,19 @@ void Engine::compileHess()
 }
 
 // The one-pass form costs the same for any number of directions, forward mode
-// a pass per direction: K+K-pi0, 11.1M events, 4.0 ms against 1.3 ms per
-// direction (30.1 ms for all 23); three chains of rho, 1.11M events, 0.51 ms
-// against 0.13 ms (3.2 ms for all 24).
+// a pass per direction, cheaper for those that move couplings alone. 1.1M
+// events, microseconds: one pass, forward mode for four coupling directions,
+// four resonance directions, all:
+//   one rho       4 rows:  122,  147,  150,   150
+//   K_S K_S       8 rows:  202,  408,  516,   797
+//   K+K-pi0      23 rows:  495,  546,  919,  3085
+//   3 chains     24 rows:  527,  576, 1035,  3189
+//                32 rows:  811,  739, 1502,  5828
+//                40 rows: 1257,  972, 2293, 10230
+//                48 rows: 1928, 1241, 3428, 16821
+// Whether a caller's directions move resonance parameters is not known on the
+// host. From four on the one pass loses at most 0.9 ms (four couplings' at 48
+// rows) and forward mode up to 2.7 ms (six at 48 rows).
 bool Engine::onePassHessian(int ndir) const { return ndir >= 4 && hessShape(gen_).blocks > 0; }
 
 // The one pass over the events and the contraction with the directions; the
