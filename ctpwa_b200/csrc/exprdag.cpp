@@ -285,7 +285,7 @@ int Graph::deriv(int n, int j)
     case Add: r = add(deriv(nd.a, j), deriv(nd.b, j)); break;
     case Sub: r = sub(deriv(nd.a, j), deriv(nd.b, j)); break;
     case Mul:
-        if (log_.count(n)) {
+        if (log_.count(n) && nd.dep != DEP_THETA) {  // (dlog of parameters alone comes from here)
             r = scaled(dlog(n, j));
         } else if (log_.count(nd.a) || log_.count(nd.b)) {
             const int s = log_.count(nd.a) ? nd.a : nd.b, x = s == nd.a ? nd.b : nd.a;
