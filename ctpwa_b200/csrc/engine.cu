@@ -15,6 +15,7 @@
 //   sample) -> ct_finalize (deterministic reduction, loss/gradient assembly,
 //   coupling-gradient transform).
 #include "engine.hpp"
+#include "pairing.hpp"
 
 #include "angular.cuh"
 
@@ -993,8 +994,8 @@ Engine::Engine(const std::string& config_path, const EngineOptions& opt) : opt_(
         bool all = !k_ang_.empty();
         for (void* k : k_ang_) all = all && k;
         if (all && npair > 0 && nplane * npair <= 32) {
-            alloc(d_pairmax_, sizeof(unsigned long long) * (2 * nplane * npair + 3));
-            CT_CUDA(cudaMemsetAsync(d_pairmax_, 0, sizeof(unsigned long long) * (2 * nplane * npair + 3), init_stream_));
+            alloc(d_pairmax_, sizeof(unsigned long long) * nplane * (2 * npair + 3));
+            CT_CUDA(cudaMemsetAsync(d_pairmax_, 0, sizeof(unsigned long long) * nplane * (2 * npair + 3), init_stream_));
         }
     }
     for (int k = 0; k < 3; ++k)
@@ -1330,17 +1331,14 @@ std::string angularSource(const std::vector<AgGroupHost>& gh, const std::vector<
     for (size_t gi = 0; gi < gh.size(); ++gi) {
         const AgGroup& A = gh[gi].g;
         const int npair = A.npol / 2;
-        // pairmax (may be null): maxima over events of
-        // |SL_{c,npol-1-q} -+ conj(SL_{c,q})| at [(c npair + q) 2 + 0 / 1] and
-        // of |SL| at [2 nplane npair], then of |Re SL| and |Im SL| of the
-        // polarisation paired with itself (the layout of ct_pair_check_kernel),
+        // pairmax (may be null): maxima over events, the layout of pairingOf,
         // accumulated by one atomic per warp and value
         o << "extern \"C\" __global__ void __launch_bounds__(128) ct_ang_" << gi
           << "(const double* __restrict__ p4, long long n, long long ld, AgTables T, double2* __restrict__ out64,\n"
              "    float2* __restrict__ out32, double* __restrict__ kin, unsigned long long* __restrict__ pairmax)\n{\n"
              "  const long long e = (long long)blockIdx.x * 128 + threadIdx.x;\n";
         if (npair > 0) {
-            o << "  double pm[" << std::max(1, 2 * A.nsl * npair) << "] = {}, big = 0.0, mid[2] = {};\n";
+            o << "  double pm[" << std::max(1, A.nsl * (2 * npair + 3)) << "] = {};\n";
             o << "  if (e < n) {\n";
         } else {
             o << "  if (e >= n) return;\n  {\n";
@@ -1433,23 +1431,22 @@ std::string angularSource(const std::vector<AgGroupHost>& gh, const std::vector<
                   << "LL * ld + e] = v; if (out32) out32[" << plane + p
                   << "LL * ld + e] = make_float2((float)v.x, (float)v.y); }\n";
             }
+            auto maximum = [&](int k, const std::string& x, const std::string& y) {
+                o << "    pm[" << k << "] = fmax(pm[" << k << "], agDist2(" << x << ", " << y << "));\n";
+            };
             if (npair > 0) {
-                for (int p = 0; p < A.npol; ++p)
-                    o << "    big = fmax(big, agDist2(c" << last << "[" << srcs[p] << "].x, c" << last << "[" << srcs[p]
-                      << "].y));\n";
+                const int k0 = 2 * A.nsl * npair + 3 * s;
+                auto value = [&](int p) { return "c" + std::to_string(last) + "[" + std::to_string(srcs[p]) + "]"; };
+                for (int p = 0; p < A.npol; ++p) maximum(k0, value(p) + ".x", value(p) + ".y");
                 if (A.npol % 2) {
-                    const std::string c = "c" + std::to_string(last) + "[" + std::to_string(srcs[npair]) + "]";
-                    o << "    mid[0] = fmax(mid[0], agDist2(" << c << ".x, 0.0)); mid[1] = fmax(mid[1], agDist2(" << c
-                      << ".y, 0.0));\n";
+                    maximum(k0 + 1, value(npair) + ".x", "0.0");
+                    maximum(k0 + 2, value(npair) + ".y", "0.0");
                 }
                 for (int q = 0; q < npair; ++q) {
-                    const std::string a = "c" + std::to_string(last) + "[" + std::to_string(srcs[q]) + "]",
-                                      b = "c" + std::to_string(last) + "[" + std::to_string(srcs[A.npol - 1 - q]) + "]";
+                    const std::string a = value(q), b = value(A.npol - 1 - q);
                     const int k = (s * npair + q) * 2;
-                    o << "    pm[" << k << "] = fmax(pm[" << k << "], agDist2(" << b << ".x - " << a << ".x, " << b << ".y + "
-                      << a << ".y));\n";
-                    o << "    pm[" << k + 1 << "] = fmax(pm[" << k + 1 << "], agDist2(" << b << ".x + " << a << ".x, " << b
-                      << ".y - " << a << ".y));\n";
+                    maximum(k, b + ".x - " + a + ".x", b + ".y + " + a + ".y");
+                    maximum(k + 1, b + ".x + " + a + ".x", b + ".y - " + a + ".y");
                 }
             }
             o << "  }\n";
@@ -1457,18 +1454,13 @@ std::string angularSource(const std::vector<AgGroupHost>& gh, const std::vector<
         o << "  }\n";
         if (npair > 0) {
             o << "  if (pairmax) {\n    const int lane = threadIdx.x & 31;\n";
-            for (int s = 0; s < A.nsl; ++s)
-                for (int q = 0; q < npair; ++q)
-                    for (int w = 0; w < 2; ++w) {
-                        const int k = (s * npair + q) * 2 + w;
-                        const int out = ((A.plane0 + s) * npair + q) * 2 + w;
-                        o << "    { const double v = sqrt(agWarpMax(pm[" << k << "])); if (lane == 0) atomicMax(pairmax + " << out
-                          << ", (unsigned long long)__double_as_longlong(v)); }\n";
-                    }
-            for (int w = 0; w < 3; ++w)
-                o << "    { const double v = sqrt(agWarpMax(" << (w == 0 ? "big" : w == 1 ? "mid[0]" : "mid[1]")
-                  << ")); if (lane == 0) atomicMax(pairmax + " << 2 * nplane * npair + w
+            auto combine = [&](int k, int out) {
+                o << "    { const double v = sqrt(agWarpMax(pm[" << k << "])); if (lane == 0) atomicMax(pairmax + " << out
                   << ", (unsigned long long)__double_as_longlong(v)); }\n";
+            };
+            for (int i = 0; i < 2 * A.nsl * npair; ++i) combine(i, 2 * A.plane0 * npair + i);
+            for (int i = 0; i < 3 * A.nsl; ++i)
+                if (i % 3 == 0 || A.npol % 2) combine(2 * A.nsl * npair + i, 2 * nplane * npair + 3 * A.plane0 + i);
             o << "  }\n";
         }
         o << "}\n\n";
@@ -1643,21 +1635,23 @@ __global__ void ct_pair_check_kernel(const double2* __restrict__ sl, long long n
                 atomicMax(out + (c * npair + q) * 2 + 1, (unsigned long long)__double_as_longlong(dn));
             }
         }
-    double m[3] = {0.0, 0.0, 0.0};
-    for (int r = 0; r < nplane * npol; ++r) {
-        const double2* __restrict__ ra = sl + (long long)r * ld;
-        const bool self = npol % 2 && r % npol == npair;
-        for (long long e = e0; e < n; e += stride) {
-            m[0] = fmax(m[0], ct_dist(ra[e].x, ra[e].y));
-            if (self) {
-                m[1] = fmax(m[1], ct_dist(ra[e].x, 0.0));
-                m[2] = fmax(m[2], ct_dist(ra[e].y, 0.0));
+    for (int c = 0; c < nplane; ++c) {
+        double m[3] = {0.0, 0.0, 0.0};
+        for (int p = 0; p < npol; ++p) {
+            const double2* __restrict__ ra = sl + (long long)(c * npol + p) * ld;
+            const bool self = npol % 2 && p == npair;
+            for (long long e = e0; e < n; e += stride) {
+                m[0] = fmax(m[0], ct_dist(ra[e].x, ra[e].y));
+                if (self) {
+                    m[1] = fmax(m[1], ct_dist(ra[e].x, 0.0));
+                    m[2] = fmax(m[2], ct_dist(ra[e].y, 0.0));
+                }
             }
         }
-    }
-    for (int w = 0; w < 3; ++w) {
-        const double v = ct_warp_max(m[w]);
-        if (lane == 0) atomicMax(out + 2 * nplane * npair + w, (unsigned long long)__double_as_longlong(v));
+        for (int w = 0; w < 3; ++w) {
+            const double v = ct_warp_max(m[w]);
+            if (lane == 0) atomicMax(out + 2 * nplane * npair + 3 * c + w, (unsigned long long)__double_as_longlong(v));
+        }
     }
 }
 
@@ -1695,19 +1689,15 @@ void Engine::pairPolarisations()
     const int npol = model_.npol, nplane = gen_.nplane, npair = npol / 2;
     const char* off = std::getenv("CTPWA_NO_POL_PAIRING");
     if (!opt_.pair_polarisations || npair == 0 || nplane * npair > 32 || (off && *off && *off != '0')) return;
-    const int nout = 2 * nplane * npair + 3;
-    std::vector<double> worst(2 * nplane * npair, 0.0);
-    double big = 0.0, mid[2] = {0.0, 0.0};
-    if (d_pairmax_) {
-        // gathered by the generated angular kernels over all three samples
-        std::vector<unsigned long long> h(nout);
-        CT_CUDA(cudaMemcpyAsync(h.data(), d_pairmax_, sizeof(unsigned long long) * nout, cudaMemcpyDeviceToHost,
-                                init_stream_));
+    const int nout = nplane * (2 * npair + 3);
+    std::vector<double> maxima(nout, 0.0);
+    auto gather = [&](const unsigned long long* d) {
+        std::vector<double> h(nout);
+        CT_CUDA(cudaMemcpyAsync(h.data(), d, sizeof(double) * nout, cudaMemcpyDeviceToHost, init_stream_));
         CT_CUDA(cudaStreamSynchronize(init_stream_));
-        for (int i = 0; i < 2 * nplane * npair; ++i) std::memcpy(&worst[i], &h[i], sizeof(double));
-        std::memcpy(&big, &h[2 * nplane * npair], sizeof(double));
-        std::memcpy(mid, &h[2 * nplane * npair + 1], 2 * sizeof(double));
-    }
+        for (int i = 0; i < nout; ++i) maxima[i] = std::max(maxima[i], h[i]);
+    };
+    if (d_pairmax_) gather(d_pairmax_);  // by the generated angular kernels over all three samples
     unsigned long long* d_out = nullptr;
     if (!d_pairmax_) alloc(d_out, sizeof(unsigned long long) * nout);
     for (int k = 0; k < 3 && !d_pairmax_; ++k) {
@@ -1717,38 +1707,17 @@ void Engine::pairPolarisations()
         const unsigned grid = (unsigned)std::min<long long>((d.n + 255) / 256, 148LL * 8);
         ct_pair_check_kernel<<<grid, 256, 0, init_stream_>>>(d.slamp64, d.n, d.ld, nplane, npol, d_out);
         CT_CUDA(cudaGetLastError());
-        std::vector<unsigned long long> h(nout);
-        CT_CUDA(cudaMemcpyAsync(h.data(), d_out, sizeof(unsigned long long) * nout, cudaMemcpyDeviceToHost, init_stream_));
-        CT_CUDA(cudaStreamSynchronize(init_stream_));
-        for (int i = 0; i < 2 * nplane * npair; ++i) {
-            double x;
-            std::memcpy(&x, &h[i], sizeof(double));
-            worst[i] = std::max(worst[i], x);
-        }
-        double b[3];
-        std::memcpy(b, &h[2 * nplane * npair], 3 * sizeof(double));
-        big = std::max(big, b[0]);
-        for (int w = 0; w < 2; ++w) mid[w] = std::max(mid[w], b[1 + w]);
+        gather(d_out);
     }
     devFree(d_out);
-    const double tol = 1e-12 * big;
-    unsigned neg = 0;
-    bool ok = big > 0.0;
-    for (int c = 0; c < nplane && ok; ++c)
-        for (int q = 0; q < npair && ok; ++q) {
-            const double dp = worst[(c * npair + q) * 2], dn = worst[(c * npair + q) * 2 + 1];
-            if (dp <= tol) continue;
-            if (dn <= tol) neg |= 1u << (c * npair + q);
-            else ok = false;
-        }
-    // the paired kernels rebuild conjugates with a plus sign
-    if (!ok || neg != 0) return;
+    const Pairing pairing = pairingOf(nplane, npol, maxima.data());
+    if (!pairing.pairs) return;
     const int ns = (npol + 1) / 2;
     // The FP64 kernels read the polarisation paired with itself as a real
     // number: parity makes it real or imaginary, in all planes alike, and a
     // phase common to a polarisation changes neither |S_p|^2 nor any gradient.
-    const bool mid_im = npol % 2 && mid[1] > tol;
-    paired_[0] = npol % 2 == 0 || mid[0] <= tol || mid[1] <= tol;
+    const bool mid_im = pairing.mid_im;
+    paired_[0] = pairing.reals;
     paired_[1] = opt_.mixed_tables;
     for (int pr = 0; pr < 2; ++pr)
         if (paired_[pr]) (pr == 0 ? k_f64_ : k_mixed_) = k_pc_[pr];
