@@ -11,7 +11,8 @@ perturbed every step, so every lineshape is recomputed.
 
     python bench.py [--gpus N] [--steps K] [--warmup W] [--impl b200|reference]
 
-One JSON line on rank 0. `value` is the mixed-precision path (FP32 angular
+One JSON line on rank 0 (stdout); everything measured, the legs beside the
+headline included, goes to stderr as one JSON line before it. `value` is the mixed-precision path (FP32 angular
 tables, lineshapes and coherent sum; FP64 logs and accumulations) with the
 events resident in HBM; the FP64 path is timed beside it; `e2e` goes through
 the host-buffer C-ABI entry point. Multi-GPU: each rank holds its own shard of
@@ -607,6 +608,27 @@ def toy_fit(args, device):
                                   "precision (ctpwa_fit_batched, 200 us gather window)"}}
 
 
+def headline(line):
+    """The line of stdout: the headline and what explains it, short enough to be read from the end of a log that keeps
+    its last 1500 characters."""
+    def short(x):
+        if isinstance(x, float):
+            return float(f"{x:.7g}")
+        return {k: short(v) for k, v in x.items()} if isinstance(x, dict) else x
+
+    out = {k: v for k, v in line.items() if not isinstance(v, dict)}
+    out["config"] = line["config"]
+    out["clocks"], out["e2e"], out["accuracy"] = line["clocks"], line["e2e"], line["accuracy"]
+    out["fp64"] = {k: line["fp64"][k] for k in ("value", "kernel_ms")}
+    out["roofline"] = {k: line["roofline"][k] for k in ("achieved", "peak", "unit", "frac", "kernel_ms")}
+    if "hessian" in line:
+        out["hessian_ms"] = line["hessian"]["exact_ms"]
+    if line.get("toy_fit", {}).get("sweep"):
+        fits = line["toy_fit"]["sweep"][0]
+        out["toy_fit_ms"] = {"p50": fits["mixed"]["fit_ms_p50"], "p99": fits["mixed"]["fit_ms_p99"]}
+    return short(out)
+
+
 def run_gpu(args, rank, world, local_rank):
     import torch
     import torch.distributed as dist
@@ -722,7 +744,7 @@ def run_gpu(args, rank, world, local_rank):
     e2e = {"value": world * E / e2e_s, "unit": UNIT, "h2d_bytes_per_step": 8 * nP, "d2h_bytes_per_step": 8 * (1 + nP),
            "ms_per_step": 1e3 * e2e_s / E}
 
-    # full-size Hessian: exact (forward mode over the adjoint pass) and
+    # full-size Hessian: exact (one pass over the events) and
     # central differences of the exact gradient, each timed once after one
     # untimed call; several GPUs: the sharded form (two all-reduces)
     hess = None
@@ -781,9 +803,8 @@ def run_gpu(args, rank, world, local_rank):
         "higher_is_better": True,
         "scaling": "weak",
         "vs_baseline": None,
-        "dtype": "f32+f64 (mixed: FP32 angular tables, lineshapes and coherent sum; FP64 m0^2-m^2, log and sums)",
-        "data": "synthetic, generated on the GPU (seeded phase space, accept-reject data, uniform background), "
-                "events resident in HBM",
+        "dtype": "f32+f64 (FP32 angular tables, lineshapes, coherent sum; FP64 m0^2-m^2, log, sums)",
+        "data": "synthetic (seeded, generated on the GPU, resident in HBM)",
         "config": workload_config() if args.fraction == 1.0 else dict(workload_config(), fraction=args.fraction),
         "run": {"events_per_rank": {"phsp": n_events[0], "data": n_events[1], "bkg": n_events[2]},
                 "n_params": nP, "launch": ana.launchShape(),
@@ -798,9 +819,9 @@ def run_gpu(args, rank, world, local_rank):
         "accuracy": {"abs_dnll_mixed_vs_fp64": dnll, "grad_rel_err_mixed_vs_fp64": grel},
         "clocks": clocks,
         "e2e": e2e,
-        # per step: prepare, prologue, fused pass, finalize
-        # (multi-GPU: + per-sample row sums and a second prepare before the finalize)
-        "gpu_launches": (4 + (2 if world > 1 else 0)) * K,
+        # per step: prologue, fused pass, finalize
+        # (multi-GPU: + per-sample row sums and the couplings before the finalize)
+        "gpu_launches": (3 + (2 if world > 1 else 0)) * K,
         "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s", "frac": achieved / peak,
                      "traffic": traffic, "peak_source": peak_src,
                      "kernel": "ct_fused_mixed",
@@ -821,7 +842,8 @@ def run_gpu(args, rank, world, local_rank):
         line["reference_cuda"] = reference_cuda_timing(args, local_rank)
     if cpu_cfg is not None:
         line["cpu_baseline"] = cpu_baseline(str(cpu_cfg), p0, n_events)
-    print(json.dumps(line), flush=True)
+    print(json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(headline(line)), flush=True)
     return 0
 
 
