@@ -824,8 +824,10 @@ class analysis:
     def getHessian(self, params: torch.Tensor, method: str = "exact", rel_step: float = 1e-5) -> torch.Tensor:
         """Hessian [(2nV+nT), (2nV+nT)] (float64, CUDA), grouped [Re p, Im p, theta].
 
-        method "exact" (default): forward-mode (dual-number) derivatives of the
-        FP64 device gradient pass along every unit direction, symmetrised.
+        method "exact" (default): FP64 first and second derivatives in one pass
+        over the events, symmetrised; models of more than 48 real parameters or
+        16 polarisation states take forward-mode (dual-number) derivatives of
+        the device gradient pass along every unit direction instead.
         method "fd": central differences of the exact FP64 device gradient with
         steps rel_step * max(|p_i|, 1e-2).
         method "gram": the coupling block from tensor-core Gram sums over the

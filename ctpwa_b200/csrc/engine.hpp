@@ -127,7 +127,7 @@ public:
     // so calls on one handle must be ordered against its other evaluations.
     void nllGradStatic(const double* d_params, double* d_nll, double* d_grad, int precision, cudaStream_t stream);
     // The evaluations of several handles of one model (same generated kernel)
-    // in one prepare, prologue, fused and finalize launch on `stream`; each
+    // in one prologue, fused and finalize launch on `stream`; each
     // job's NLL and gradient equal its own nllGrad's. Device pointers per job.
     // Identity of the compiled fused kernel image (generated model and
     // launch layout): handles with equal keys can share a multi-job launch.

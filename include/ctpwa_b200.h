@@ -143,9 +143,11 @@ int ctpwa_hessian(ctpwa_handle* h, const double* d_params, double* d_hess, doubl
  * computeDataHessianContribFast, computePhspHessian, computeUnifiedHessian and
  * transformExtendedHessian, src/ComputeHessian.cu:149-1556,
  * src/AmpGen.cu:3020-3540, src/Parameters.cu:348-584).
- * The exact FP64 Hessian, same layout as ctpwa_hessian: forward-mode
- * (dual-number) derivatives of the device gradient pass along the n_params
- * unit directions, symmetrised. The first call on a handle compiles the
+ * The exact FP64 Hessian, same layout as ctpwa_hessian, symmetrised: in one
+ * pass over the events for models of at most 48 real parameters (amplitude
+ * couplings and free resonance parameters) and 16 polarisation states, else by
+ * forward-mode (dual-number) derivatives of the device gradient pass along the
+ * n_params unit directions. The first call on a handle compiles the
  * kernels (or loads them from the kernel cache) and allocates their buffers;
  * later calls are queued on the stream without host synchronisation. */
 int ctpwa_hessian_exact(ctpwa_handle* h, const double* d_params, double* d_hess, void* stream);
