@@ -1934,13 +1934,15 @@ FusedShape fusedShape(const GeneratedModel& gen)
     // sums fit. Sums in registers spill: three chains of 7 resonances, 77 sums
     // (2.2M events, whole evaluations), 921 us at 192 against 322 us at 128 in
     // shared memory; 8 resonances 1224 and 361 us; 6 resonances 335 us at 192
-    // without the copies, 293 us at 128 with them. Paired: three chains of rho 5.55M events 0.262 ms against
-    // 0.287 ms, K_S K_S 1.1M events 0.045 against 0.047 ms; K+K-pi0 has room
-    // for 192 only (256 with direct loads 0.61 ms against 0.56 ms). Unpaired
-    // (whole evaluations): three chains of rho have room for 192, 0.353 ms
-    // against 0.399 ms with direct loads at 256; one chain 41 us at 256 and 42
-    // at 192, K_S K_S 77 and 74 us; K+K-pi0 5.5M events 0.372 ms at 128 against
-    // 0.449 ms with direct loads at 192.
+    // without the copies, 293 us at 128 with them.
+    // Paired: three chains of rho 5.55M events 0.262 ms at 256 against 0.287 ms
+    // at 192, K_S K_S 1.1M events 0.045 against 0.047 ms; K+K-pi0 has room for
+    // 192 (256 with direct loads 0.61 ms against 0.56 ms; whole evaluations of
+    // 5.5M events 301 us at 192, 311 us at 128).
+    // Unpaired (whole evaluations): three chains of rho have room for 192,
+    // 0.353 ms against 0.399 ms with direct loads at 256; one chain 41 us at
+    // 256 and 42 at 192, K_S K_S 77 and 74 us; K+K-pi0 5.5M events 0.372 ms at
+    // 128 against 0.449 ms with direct loads at 192.
     auto f64_block = [&](int paired) {
         for (int b : {256, 192, kPlainBlockMin})
             if (fits(0, sums(0, b) + staged[paired] * b)) return b;
